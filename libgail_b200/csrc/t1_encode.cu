@@ -15,12 +15,10 @@
 // Stage 2, ordering (t1OrderKernel): counting sort of the blocks by decision count, most
 // first, so the longest serial MQ chains start first.
 //
-// Stage 3, MQ coding (t1MqKernel): one lane per code-block. Lanes pull blocks from a
-// device queue one at a time, so a lane that finishes early takes the next block
-// instead of idling while its warp-mates finish. The coder is in branch-free
-// select form (both MPS and LPS take the same instruction path until renormalisation),
-// its contexts live in shared memory, and its input is prefetched 16 decisions ahead.
-// The MQ state at each pass's end is recorded.
+// Stage 3, MQ coding (t1MqKernel): one lane per code-block; a warp takes the next 32 blocks
+// of the order at once. The coder takes 16 decisions at a time in branch-free select form,
+// then the bytes they completed; its contexts live in shared memory, and its input is
+// loaded 32 decisions ahead. The MQ state at each pass's end is recorded.
 //
 // Stage 4, truncation lengths (t1TruncKernel): a warp per block, a lane per pass; each
 // pass's length is found from its recorded MQ state and the final codeword bytes. Kept
@@ -465,19 +463,31 @@ __global__ void __launch_bounds__(256) t1OrderScatterKernel(T1Launch P) {
 }
 
 // ---------------------------------------------------------------------------- MQ coding
-// Context state word: Qe | MPS << 16 | state index << 17. nextStateEntry(k), k = state
-// index << 2 | MPS << 1 | LPS: the state word after a renormalising decision; the coder keeps
-// the two entries of each (state, MPS) side by side.
-__device__ __forceinline__ uint32_t nextStateEntry(uint32_t k) {
-    const uint32_t idx = k >> 2, mps = (k >> 1) & 1u, lps = k & 1u, e = c_mq[idx];
-    const uint32_t nidx = lps ? (e >> 24) & 63u : (e >> 18) & 63u;
-    const uint32_t nm = mps ^ (lps ? (e >> 17) & 1u : 0u);
-    return (c_mq[nidx] & 0xFFFFu) | (nm << 16) | (nidx << 17);
-}
-__device__ __forceinline__ uint32_t initialState(uint32_t idx) { return (c_mq[idx] & 0xFFFFu) | (idx << 17); }
+// The layout of a lane's MQ memory: 20 context states (19 contexts and the null context, whose
+// decisions change nothing) and a round's 16 steps, word i of either CS words after word i - 1. A
+// decision byte is context << 1 | bit; CS is such that the context's byte offset is the byte
+// shifted left by SHIFT, its bit masked off.
+template <int CS>
+struct MqLayout {
+    static_assert(CS == 32 || CS == 128, "context stride");
+    static constexpr int SHIFT = CS == 128 ? 8 : 6;
+    static constexpr uint32_t kCtxMask = 0x3Eu << SHIFT;
+    // Context state word: Qe << 16 | the byte offset of its successors, in which bit SHIFT is the
+    // MPS (where a decision byte shifted left by SHIFT has its bit) and the state index fills
+    // the other bits from 3 on.
+    __device__ static uint32_t word(uint32_t idx, uint32_t mps) {
+        const uint32_t low = idx & ((1u << (SHIFT - 3)) - 1u), high = idx >> (SHIFT - 3);
+        const uint32_t qe = c_mq[idx] << 16;
+        return qe | ((uint32_t)__clz((int)qe) << 10) | (high << (SHIFT + 1)) | (mps << SHIFT) | (low << 3);
+    }
+};
+constexpr uint32_t kOffMask = 0x3F8u;   // the successors' offset in a state word
+constexpr uint32_t kNullByte = 19u << 1;  // a decision in the null context (state word 0)
+constexpr int MQ_CTX = 20, MQ_ROUND = 16, MQ_WORDS = MQ_CTX + MQ_ROUND;
 
+// The code register of one block: the interval's base, the bits shifted out of it, the bytes.
 struct Coder {
-    uint32_t A, C, B;
+    uint32_t C, B;
     int CT, bp;
     uint8_t* out;
     uint32_t cap;
@@ -499,34 +509,8 @@ struct Coder {
         C &= stuff ? 0xFFFFFu : 0x7FFFFu;
         CT = stuff ? 7 : 8;
     }
-    // One decision in context state t; returns the context's next state. Renormalisation
-    // shifts by clz(A) - 16, which is 0 when A stayed at or above 0x8000; the byte-out is the
-    // only branch. next[t >> 16] holds both successors of the state (after an MPS that
-    // renormalises, after an LPS), so the load does not wait for the decision's outcome.
-    __device__ __forceinline__ uint32_t encode(uint32_t t, uint32_t d, const uint2* next) {
-        const uint2 succ = next[t >> 16];
-        const uint32_t qe = t & 0xFFFFu;
-        const uint32_t a = A - qe;
-        const bool lps = ((d ^ (t >> 16)) & 1u) != 0;
-        const bool upper = (a >= qe) != lps;  // which sub-interval the decision takes
-        C += upper ? qe : 0u;
-        A = upper ? a : qe;
-        const bool rn = lps || !(a & 0x8000u);
-        const uint32_t nt = lps ? succ.y : succ.x;
-        int n = __clz(A) - 16;
-        A <<= n;
-        for (;;) {
-            const int sh = min(n, CT);
-            C <<= sh;
-            CT -= sh;
-            n -= sh;
-            if (CT != 0) break;
-            byteout();
-            if (n == 0) break;
-        }
-        return rn ? nt : t;
-    }
-    __device__ __forceinline__ uint32_t flush() {
+    // A: the interval, 16 bits
+    __device__ __forceinline__ uint32_t flush(uint32_t A) {
         const uint32_t tempc = C + A;
         C |= 0xFFFFu;
         if (C >= tempc) C -= 0x8000u;
@@ -597,33 +581,57 @@ __device__ uint32_t truncLen(uint4 s, const uint8_t* buf, uint32_t len, uint32_t
     return len;
 }
 
+// s_next: by a state word's offset, its successors after an MPS that renormalises and after an
+// LPS; s_init: the initial state words of Table D.7 (ZC context 0 state 4, run-length 3,
+// uniform 46, every other 0).
+template <int CS>
 __device__ __forceinline__ void mqTables(uint2* s_next, uint32_t* s_init) {
-    for (int i = threadIdx.x; i < 2 * 47; i += blockDim.x)
-        s_next[i] = make_uint2(nextStateEntry(2 * i), nextStateEntry(2 * i + 1));
+    using M = MqLayout<CS>;
+    for (int i = threadIdx.x; i < 2 * 47; i += blockDim.x) {
+        const uint32_t idx = i >> 1, mps = i & 1u, e = c_mq[idx];
+        s_next[(M::word(idx, mps) & kOffMask) >> 3] =
+            make_uint2(M::word((e >> 18) & 63u, mps), M::word((e >> 24) & 63u, mps ^ ((e >> 17) & 1u)));
+    }
     if (threadIdx.x == 0) {
-        s_init[0] = initialState(0);
-        s_init[1] = initialState(4);
-        s_init[2] = initialState(3);
-        s_init[3] = initialState(46);
+        s_init[0] = M::word(0, 0);
+        s_init[1] = M::word(4, 0);
+        s_init[2] = M::word(3, 0);
+        s_init[3] = M::word(46, 0);
     }
 }
 
-// MQ coding, a lane per block, until the queue is empty. ctx: the lane's 19 context states,
-// CS words apart. warpId: the warp's place among the solo warps of a separate MQ launch.
-// PERS (a persistent launch): the solo blocks go to the first warps to get here, and each
-// block, coded or empty, is listed for its truncation lengths when it is done.
-template <int CS, bool PERS>
-__device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* ctx, const uint2* s_next, const uint32_t* s_init,
-                                      uint32_t warpId) {
+// MQ coding, a lane per block, until the queue is empty. s_mq: the CTA's MQ memory (MqLayout),
+// lane0: this lane's first word in it. warpId: the warp's place among the solo warps of a
+// separate MQ launch. PERS (a persistent launch): the solo blocks go to the first warps to get
+// here, and each block, coded or empty, is listed for its truncation lengths when it is done.
+//
+// Bound by the serial chain of a block's decisions (one-frame launches) or by instruction
+// issue (batched ones). 16 decisions are a straight line of code without a branch: decisions
+// outside the lane's pass (before its position, after the pass's end) count as decisions in the
+// null context, so every lane of the warp takes the same 16 steps. The bytes are taken out
+// after them, where a byte completed in the middle of a decision made nearly every decision
+// of a warp take the byte's branch as well. A round sets up 32 decisions (16 at a time: 3-5 %
+// slower). On a B200, per 4K frame (154 M decisions): 1.11 ms alone where the coder with the
+// branch took 2.21, 0.50 ms of a batch of eight; the 48 blocks of a 64 x 64 frame 0.48 ms,
+// where they took 1.35. CHAIN: the form with the shorter chain and a few more instructions,
+// for one-frame launches (1.15 against 1.18 ms).
+template <int CS, bool PERS, bool CHAIN>
+__device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* s_mq, uint32_t lane0, const uint2* s_next,
+                                      const uint32_t* s_init, uint32_t warpId) {
+    using M = MqLayout<CS>;
     uint32_t* status = P.ctl + 1;
     const int lane = threadIdx.x & 31;
+    uint8_t* const ctxBytes = reinterpret_cast<uint8_t*>(s_mq);
+    uint32_t* const steps = s_mq + MQ_CTX * CS + lane0;
+    const uint32_t laneByte = 4u * lane0;
+    auto ctxAt = [&](uint32_t off) -> uint32_t& { return *reinterpret_cast<uint32_t*>(ctxBytes + off); };
 
-    // Per-lane state of the block in hand. Invariant between decisions: s is the decision
-    // at pos and t the state of its context; nxt holds the decisions from pos on.
-    uint32_t job = 0, pos = 0, nsym = 0, np = 0, k = 0, nextEnd = 0, stop = 0, s = 0, t = 0;
+    // Per-lane state of the block in hand: the interval A (in the upper half), the next decision
+    // (pos), the 32 decisions around it (cur) and after those (nxt).
+    uint32_t job = 0, pos = 0, nsym = 0, np = 0, k = 0, nextEnd = 0, A = 0;
     uint32_t laterEnd = 0;  // the pass end after nextEnd, loaded one pass ahead
     const uint8_t* sym = nullptr;
-    uint4 nxt = make_uint4(0, 0, 0, 0);
+    uint4 cur[2], nxt[2];
     Coder e;
     e.cap = 0;
     bool have = false;
@@ -635,7 +643,28 @@ __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* ctx, const ui
             atomicExch(P.work + kWList + slot, j + 1);
         }
     };
-    // starts block j; false when it has no coding pass (nothing to code)
+    auto load = [&](uint32_t at) {
+        return at < nsym ? ldx<false>(reinterpret_cast<const uint4*>(sym + at)) : make_uint4(0, 0, 0, 0);
+    };
+    // the MQ state at every pass end the position has reached; false when the block is done
+    auto passEnds = [&] {
+        while (k < np && pos == nextEnd) {
+            P.snaps[(size_t)job * kMaxPasses + k] =
+                make_uint4((uint32_t)e.bp, e.C, (A >> 16) | ((uint32_t)e.CT << 16), e.B);
+            ++k;
+            nextEnd = laterEnd;  // loaded a pass ago: no wait here
+            laterEnd = k + 1 < np ? ldx<false>(P.passEnd + (size_t)job * kMaxPasses + k + 1) : 0xFFFFFFFFu;
+        }
+        if (k < np) return true;
+        // flush, and the codeword's length (the truncation lengths are found afterwards, a
+        // warp per block)
+        const uint32_t len = e.flush(A >> 16);
+        if (e.overflow) atomicOr(status, kErrCodewordSpace);
+        P.info[4 * (size_t)job + 3] = e.overflow ? 0u : len;
+        listed(job);
+        return false;
+    };
+    // starts block j; false when there is nothing (more) to code
     auto begin = [&](uint32_t j) {
         job = j;
         np = ldx<false>(P.info + 4 * (size_t)job + 1);
@@ -649,28 +678,133 @@ __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* ctx, const ui
         sym = J.sym;
         e.out = J.cw;
         e.cap = J.cap;
-        e.A = 0x8000u;
+        A = 0x80000000u;
         e.C = 0;
         e.CT = 12;
         e.bp = -1;
         e.B = 0;
         e.overflow = false;
-        // initial states, Table D.7: ZC context 0 state 4, run-length 3, uniform 46
 #pragma unroll
-        for (int c = 0; c < 19; ++c) ctx[c * CS] = s_init[0];
-        ctx[0] = s_init[1];
-        ctx[17 * CS] = s_init[2];
-        ctx[18 * CS] = s_init[3];
+        for (int c = 0; c < 19; ++c) s_mq[c * CS + lane0] = s_init[c == 0 ? 1 : c == 17 ? 2 : c == 18 ? 3 : 0];
+        s_mq[19 * CS + lane0] = 0u;
         pos = 0;
         k = 0;
         nextEnd = ldx<false>(P.passEnd + (size_t)job * kMaxPasses);
         laterEnd = np > 1 ? ldx<false>(P.passEnd + (size_t)job * kMaxPasses + 1) : 0xFFFFFFFFu;
-        stop = min(nsym, nextEnd);
-        nxt = nsym ? ldx<false>(reinterpret_cast<const uint4*>(sym)) : make_uint4(0, 0, 0, 0);
-        s = nxt.x & 0xFFu;
-        t = ctx[(s >> 1) * CS];
-        have = true;
-        return true;
+        cur[0] = load(0);
+        cur[1] = load(16);
+        nxt[0] = load(32);
+        nxt[1] = load(48);
+        return passEnds();
+    };
+    // 16 decisions, those outside the pass in the null context
+    auto steps16 = [&](const uint4& c) {
+        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+        // decision b of the round shifted left by SHIFT (its other bytes beside it)
+        auto shifted = [&](int b) {
+            const int sh = 8 * (b & 3) - M::SHIFT;
+            return sh >= 0 ? w[b >> 2] >> sh : w[b >> 2] << -sh;
+        };
+        uint32_t v = shifted(0), at = (v & M::kCtxMask) | laneByte, t = ctxAt(at);
+        unsigned long long code = e.C;  // the code register with the round's shifts
+        uint32_t shift = 0;
+#pragma unroll
+        for (int b = 0; b < MQ_ROUND; ++b) {
+            const uint32_t vNext = b < MQ_ROUND - 1 ? shifted(b + 1) : 0u, atNext = (vNext & M::kCtxMask) | laneByte;
+            const uint32_t ahead = b < MQ_ROUND - 1 ? ctxAt(atNext) : 0u;  // unless this decision changes it
+            const uint2 succ = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(s_next) + (t & kOffMask));
+            const uint32_t qe = t & 0xFFFF0000u, a = A - qe;
+            const bool lps = ((v ^ t) & (1u << M::SHIFT)) != 0;
+            const bool upper = (a >= qe) != lps;  // which sub-interval the decision takes
+            const uint32_t q = upper ? qe : 0u;
+            uint32_t n;
+            if constexpr (CHAIN) {
+                // the shift without a count of leading zeros, whose latency is most of the chain:
+                // Qe's is in the state word, and what is left of the interval needs two at most
+                const uint32_t nq = (t >> 10) & 15u;
+                const uint32_t lowerA = qe << nq;
+                const bool p1 = (int)a >= 0, p2 = a < 0x40000000u;
+                const uint32_t upperA = p2 ? a << 2 : p1 ? a << 1 : a;
+                A = upper ? upperA : lowerA;
+                n = upper ? (p2 ? 2u : p1 ? 1u : 0u) : nq;
+            } else {
+                A = upper ? a : qe;
+                n = (uint32_t)__clz((int)A);
+                A <<= n;
+            }
+            const uint32_t renormed = lps ? succ.y : succ.x;
+            const uint32_t after = lps || (int)a >= 0 ? renormed : t;  // renormalises: a below 0x8000, or the LPS
+            ctxAt(at) = after;
+            steps[b * CS] = q | n;
+            code = (code + (q >> 16)) << n;
+            shift += n;
+            t = atNext == at ? after : ahead;
+            at = atNext;
+            v = vNext;
+        }
+        // The bytes the round completed, all from the register as it stands after the round. At
+        // its own time a byte had not yet the carry of what was added since: the same byte
+        // comes out one higher at once instead of at the next byte, except an 0xFF, after which
+        // the coder keeps room for the carry instead of passing it on. A byte that may have been
+        // one (it and the three bits below read 0 after a carry), and a round of more shifts
+        // than the register holds, are done over from the steps, byte by byte.
+        const Coder before = e;
+        int left = (int)shift;
+        bool redo = shift > 32u;
+        uint32_t keep = 0xFFFFFFFFu;
+        while (left >= e.CT) {
+            left -= e.CT;
+            e.C = (uint32_t)(code >> left) & keep;
+            redo = redo || (e.C & 0x7FF0000u) == 0u;
+            e.byteout();
+            keep = 0x7FFFFFFu;
+        }
+        e.CT -= left;
+        e.C = (uint32_t)code;
+        if (keep != 0xFFFFFFFFu) e.C &= (1u << (27 - e.CT)) - 1u;
+        if (redo) {
+            e = before;
+#pragma unroll 1
+            for (int b = 0; b < MQ_ROUND; ++b) {
+                const uint32_t x = steps[b * CS];
+                e.C += x >> 16;
+                int n = (int)(x & 31u);
+                while (n >= e.CT) {
+                    e.C <<= e.CT;
+                    n -= e.CT;
+                    e.byteout();
+                }
+                e.C <<= n;
+                e.CT -= n;
+            }
+        }
+    };
+
+    // the decisions from pos to the end of its 32 or of its pass
+    auto round = [&] {
+        const uint32_t first = pos & ~31u, lo = pos & 31u, hi = min(32u, nextEnd - first);
+        uint4 c0 = cur[0], c1 = cur[1];
+        const uint32_t in = (hi == 32u ? kFull : (1u << hi) - 1u) & ~((1u << lo) - 1u);
+        if (in != kFull) {
+            uint32_t* const w[8] = {&c0.x, &c0.y, &c0.z, &c0.w, &c1.x, &c1.y, &c1.z, &c1.w};
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t m = spread1((in >> (4 * q)) & 0xFu) * 0xFFu;
+                *w[q] = (*w[q] & m) | (kNullByte * 0x01010101u & ~m);
+            }
+        }
+        pos = first + hi;
+        if (hi == 32u) {
+            cur[0] = nxt[0];
+            cur[1] = nxt[1];
+            nxt[0] = load(pos + 32u);
+            nxt[1] = load(pos + 48u);
+        }
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            if ((in >> (16 * half)) & 0xFFFFu) steps16(c0);
+            c0 = c1;
+        }
     };
 
     // A solo warp first codes its solo block (perm[0 .. solo)) on its lane 0 while the other
@@ -685,105 +819,39 @@ __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* ctx, const ui
         if (lane == 0) mine = atomicAdd(P.work + kWSoloHead, 1u);
         mine = __shfl_sync(kFull, mine, 0);
     }
-    // end of the block in hand: remaining pass ends, flush, the codeword's length (the
-    // truncation lengths are found afterwards, a warp per block)
-    auto endBlock = [&] {
-        while (k < np) {
-            P.snaps[(size_t)job * kMaxPasses + k] = make_uint4((uint32_t)e.bp, e.C, e.A | ((uint32_t)e.CT << 16), e.B);
-            ++k;
-        }
-        const uint32_t len = e.flush();
-        if (e.overflow) atomicOr(status, kErrCodewordSpace);
-        P.info[4 * (size_t)job + 3] = e.overflow ? 0u : len;
-        listed(job);
-        have = false;
-    };
-    // one aligned chunk of 16 decisions of the block in hand (fewer at its end)
-    auto chunk = [&] {
-        // one aligned chunk of 16 decisions (fewer at the block's end): a word of four
-        // decisions unrolled at a time, the next decision's context state read ahead, off
-        // the serial chain of the coder
-        const uint4 v = nxt;
-        nxt = (pos + 16 < nsym) ? ldx<false>(reinterpret_cast<const uint4*>(sym + pos + 16)) : make_uint4(0, 0, 0, 0);
-        uint32_t w0 = v.x, w1 = v.y, w2 = v.z, w3 = v.w;
-        const uint32_t w4 = nxt.x;
-        // one decision: s (context and bit) in state t; sn the next decision
-        auto one = [&](uint32_t sn) {
-            // the byte past the block's last decision is not a decision: the clamp keeps its
-            // look-ahead read inside the lane's 19 contexts
-            const uint32_t cn = min(sn >> 1, 18u), cx = s >> 1;
-            const uint32_t tn = ctx[cn * CS];
-            const uint32_t tNew = e.encode(t, s & 1u, s_next);
-            ctx[cx * CS] = tNew;
-            t = cn == cx ? tNew : tn;
-            s = sn;
-            ++pos;
-        };
-        bool done = false;
-#pragma unroll 1
-        for (int q = 0; q < 4 && !done; ++q) {
-            const uint32_t cur = w0;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (pos >= stop) {
-                    if (pos >= nsym) {
-                        done = true;
-                        break;
-                    }
-                    while (pos == nextEnd && k < np) {  // pass ends before this decision
-                        P.snaps[(size_t)job * kMaxPasses + k] =
-                            make_uint4((uint32_t)e.bp, e.C, e.A | ((uint32_t)e.CT << 16), e.B);
-                        ++k;
-                        nextEnd = laterEnd;  // loaded a pass ago: no wait here
-                        laterEnd = k + 1 < np ? ldx<false>(P.passEnd + (size_t)job * kMaxPasses + k + 1) : 0xFFFFFFFFu;
-                    }
-                    stop = min(nsym, nextEnd);
-                }
-                one(b < 3 ? (cur >> (8 * (b + 1))) & 0xFFu : w1 & 0xFFu);
-            }
-            w0 = w1;
-            w1 = w2;
-            w2 = w3;
-            w3 = w4;
-        }
-    };
-    if (mine < solo) {  // warp-uniform
-        if (lane == 0) have = begin(ldx<false>(P.perm + mine));
-        while (__shfl_sync(kFull, (int)have, 0)) {
-            if (lane == 0) {
-                if (pos >= nsym) endBlock();
-                else chunk();
-            }
-        }
-    }
+    bool alone = mine < solo;  // warp-uniform
     for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(P.ctl, 32u);
-        base = __shfl_sync(kFull, base, 0);
-        if (solo + base >= P.n) break;  // warp-uniform
-        const uint32_t qi = solo + base + lane;
-        have = qi < P.n && begin(ldx<false>(P.perm + qi));
+        if (alone) {
+            have = lane == 0 && begin(ldx<false>(P.perm + mine));
+            alone = false;
+        } else {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(P.ctl, 32u);
+            base = __shfl_sync(kFull, base, 0);
+            if (solo + base >= P.n) break;  // warp-uniform
+            const uint32_t qi = solo + base + lane;
+            have = qi < P.n && begin(ldx<false>(P.perm + qi));
+        }
         while (__any_sync(kFull, have)) {
             if (have) {
-                if (pos >= nsym) endBlock();
-                else chunk();
+                round();
+                if (pos == nextEnd) have = passEnds();
             }
         }
     }
 }
 
 // MINB: CTAs per SM the registers must allow. A launch of a frame or two has fewer lanes
-// than the GPU holds and runs uncapped; wide batched launches run at 10 CTAs per SM (the
-// registers that allows need no spill; measured faster on B200 than 12 with a spill).
+// than the GPU holds and runs uncapped; wide batched launches run at 6 CTAs per SM (24 frames
+// of 4K served on a B200: 33.6 ms, 34.3 at 8 CTAs; 10 would spill).
 template <int MINB>
 __global__ void __launch_bounds__(MQ_THREADS, MINB) t1MqKernel(T1Launch P) {
-    __shared__ uint2 s_next[2 * 47];  // by (state, MPS): next state after an MPS renormalisation, after an LPS
+    __shared__ uint2 s_next[128];
     __shared__ uint32_t s_init[4];
-    __shared__ uint32_t s_ctx[19 * MQ_THREADS];
-    mqTables(s_next, s_init);
+    __shared__ uint32_t s_mq[MQ_WORDS * MQ_THREADS];
+    mqTables<MQ_THREADS>(s_next, s_init);
     __syncthreads();
-    mqRun<MQ_THREADS, false>(P, s_ctx + threadIdx.x, s_next, s_init,
-                             blockIdx.x * (MQ_THREADS / 32) + (threadIdx.x >> 5));
+    mqRun<MQ_THREADS, false, MINB == 1>(P, s_mq, threadIdx.x, s_next, s_init, blockIdx.x * (MQ_THREADS / 32) + (threadIdx.x >> 5));
 }
 
 // Truncation lengths of one block by one warp: lane q finds the shortest prefix for pass q
@@ -894,13 +962,13 @@ __global__ void __launch_bounds__(CM_THREADS, 7) t1PersistentKernel(T1Launch P, 
     };
     union WarpMem {
         WarpCm cm;
-        uint32_t ctx[19 * 32];
+        uint32_t mq[MQ_WORDS * 32];
     };
     __shared__ __align__(16) WarpMem s_w[CM_WARPS];
     __shared__ uint32_t s_hist[CM_WARPS][19];
-    __shared__ uint2 s_next[2 * 47];
+    __shared__ uint2 s_next[128];
     __shared__ uint32_t s_init[4];
-    mqTables(s_next, s_init);
+    mqTables<32>(s_next, s_init);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t* work = P.work;
@@ -956,7 +1024,7 @@ __global__ void __launch_bounds__(CM_THREADS, 7) t1PersistentKernel(T1Launch P, 
     if (!warpWaitFor(work + kWScatDone, chunks, status, lane)) return;
     // (3) MQ coding, the lanes' contexts in the warp's modelling memory
     __syncwarp();
-    mqRun<32, true>(P, s_w[wid].ctx + lane, s_next, s_init, 0);
+    mqRun<32, true, false>(P, s_w[wid].mq, (uint32_t)lane, s_next, s_init, 0);
     __syncwarp();
     // (4) truncation lengths, the list's entries in turn (an entry not yet written belongs
     // to a block whose MQ coding a running lane holds)
@@ -1061,11 +1129,21 @@ void t1Encode(const T1Launch& launch, cudaStream_t st, cudaEvent_t* marks) {
     const uint32_t cmBlocks = min(divUp(L.n, CM_WARPS), (uint32_t)sms * L.cmCtasPerSm);
     t1CmKernel<<<cmBlocks, CM_THREADS, 0, st>>>(L);
     if (marks) GB_CHECK(cudaEventRecord(marks[0], st));
-    // a wide (batched) launch gives each lane two blocks on average, so that lanes whose
-    // blocks end early take more from the queue
+    // A wide (batched) launch gives each lane two blocks on average, so that lanes whose
+    // blocks end early take more from the queue.
     const bool wide = divUp(L.n, MQ_THREADS) > (uint32_t)sms * 4u;
-    const uint32_t mqBlocks = min(divUp(L.n, MQ_THREADS * (wide ? 2u : 1u)), (uint32_t)sms * L.mqCtasPerSm);
-    const uint32_t maxSolo = mqBlocks * (MQ_THREADS / 32) / 2;
+    uint32_t mqBlocks = min(divUp(L.n, MQ_THREADS * (wide ? 2u : 1u)), (uint32_t)sms * L.mqCtasPerSm);
+    uint32_t maxSolo = mqBlocks * (MQ_THREADS / 32) / 2;
+    // A launch that does not fill one warp per scheduler is bound by its longest blocks: it
+    // gets that many warps, and as many of the longest blocks as leave a lane for every other
+    // block are coded alone (105 cycles a decision against 150 beside 31 others; a second warp
+    // on the scheduler costs a third more).
+    const uint32_t warps = (uint32_t)sms * 4u;
+    if (L.n <= warps * 32u) {
+        mqBlocks = max(mqBlocks, min(divUp(L.n, MQ_THREADS / 32), warps / (MQ_THREADS / 32)));
+        maxSolo = (warps * 32u - L.n) / 31u;
+        L.soloDecisions = 1;
+    }
     if (L.work) {  // over the whole GPU: a batch of frames has 100,000 blocks and more
         const uint32_t og = min(divUp(L.n, 256u), (uint32_t)sms * 2u);
         GB_CHECK(cudaMemsetAsync(L.work, 0, kT1WorkHead * 4, st));
@@ -1077,7 +1155,7 @@ void t1Encode(const T1Launch& launch, cudaStream_t st, cudaEvent_t* marks) {
     }
     if (marks) GB_CHECK(cudaEventRecord(marks[1], st));
     if (!wide) t1MqKernel<1><<<mqBlocks, MQ_THREADS, 0, st>>>(L);
-    else t1MqKernel<10><<<mqBlocks, MQ_THREADS, 0, st>>>(L);
+    else t1MqKernel<6><<<mqBlocks, MQ_THREADS, 0, st>>>(L);
     t1TruncKernel<<<min(divUp(L.n, (uint32_t)(TRUNC_THREADS / 32)), (uint32_t)sms * 8u), TRUNC_THREADS, 0, st>>>(L);
     GB_CHECK(cudaGetLastError());
 }
