@@ -164,6 +164,7 @@ ColorTables buildColorTables(const GailCudaColor& c) {
         }
         t.eotf[i] = (float)nits;
     }
+    t.bounded = std::all_of(t.eotf.begin(), t.eotf.end(), [](float v) { return std::fabs(v) < 1e30f; });
     double M[9];
     rgbToXyz(c.primaries, M);
     for (int i = 0; i < 9; ++i) t.m[i] = (float)M[i];
@@ -245,6 +246,9 @@ PlanarParams planarParams(const GbFrameFormat& f) {
     p.chroma = f.chroma;
     p.maxv = (float)((1 << f.bits) - 1);
     p.scale = (float)(1 << (f.bits - 8));
+    p.rMaxv = 1.0f / p.maxv;
+    p.rLuma = 1.0f / (219.f * p.scale);
+    p.rChroma = 1.0f / (224.f * p.scale);
     const double kg = 1.0 - f.kr - f.kb;
     p.crR = (float)(2 * (1 - f.kr));
     p.cbB = (float)(2 * (1 - f.kb));

@@ -41,6 +41,8 @@ struct ColorTables {
     ToneParams tone{};
     std::vector<float> lut3;  // route 2: lutN^3 nodes of three floats, red fastest
     int32_t lutN = 0;
+    // every linear value and every X, Y, Z the matrix makes of them is finite, far from overflow
+    bool bounded = false;
 };
 
 // Builds the tables of a colour setting (a 3D LUT given by path is read here). Throws
@@ -61,6 +63,7 @@ int dciCode(float n);
 struct PlanarParams {
     int32_t width, height, aw, ah, ox, oy, cw, ch, sx, sy, bits, fullRange, rgb, chroma;
     float maxv, scale, crR, cbG, crG, cbB;
+    float rMaxv, rLuma, rChroma;  // reciprocals of maxv, 219 scale and 224 scale
 };
 PlanarParams planarParams(const GbFrameFormat& f);
 // Bytes of one input frame of this format (FrameFormat::bytes, core/color.h:56-60).

@@ -268,6 +268,7 @@ void EncoderSlot::enqueueStages(const void* dFrame, bool taps, bool full) {
     c.tone = color_.tone;
     c.lut3 = dLut_;
     c.lutN = color_.lutN;
+    c.bounded = color_.bounded;
     c.xyz = taps ? dXyz_ : nullptr;
     launchFrontEnd(L_, c, dLL_[0], dLL_[1], z_.llFloats, dCoeffs_, full ? dTap_ : nullptr, st);
     GB_CHECK(cudaEventRecord(ev_[2], st));

@@ -271,6 +271,7 @@ int EncodeEngine::addClass(const GailCudaLayout& layout, const GailCudaEncodeSet
     a.tone = c->color.tone;
     a.lut3 = c->dLut;
     a.lutN = c->color.lutN;
+    a.bounded = c->color.bounded;
     const uint64_t n = c->z.n, npix = c->z.npix;
     c->dataCap = c->z.outCap;
     c->slotBytes = c->z.inBytes + n * kCblkArea * 4 + n * sizeof(T1Job) + n * 20 + n * kMaxPasses * (4 + 1 + 8) +

@@ -47,6 +47,7 @@ struct ColorArgs {
     ToneParams tone;         // route 1
     const float* lut3;       // route 2: lutN^3 nodes of three floats, red fastest
     int32_t lutN;
+    bool bounded;            // ColorTables::bounded
 };
 
 // Level 1 with the colour conversion folded into its tile loads; shape: the tile, 0 = 64 x
