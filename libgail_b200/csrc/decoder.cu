@@ -1,23 +1,14 @@
 // Decoder on sm_100a: Tier-1 decoding with dequantisation, inverse 9/7 wavelet, inverse
 // ICT and 12-bit packing.
 //
-// Tier-1 (decodeKernel): one code-block per warp at a time, decoded by its lane 0 (the
-// decode's control flow depends on every decoded bit, so lanes of one warp decoding
-// different blocks would only run one after another); up to 32 such warps per SM pull
+// Tier-1 (decodeKernel): one code-block per warp at a time; up to 24 such warps per SM pull
 // blocks from a device queue ordered longest codeword first (orderKernel), the heaviest
-// on SMs of their own. A block's state is kept as row masks in shared memory
-// (significance and sign for rows -1..32, coded-this-plane and refined); the scan visits
-// only columns that have something to code (bit scans over candidate masks) with the rows
-// above, at and below the sample in registers (one shared load per sample), zero-coding
-// and sign contexts come from shared tables keyed by the neighbour bits, the refinement
-// pass keeps its three contexts in registers, and the decoded words (sign, twice the
-// magnitude plus the mid-point of the planes not decoded) are built in shared memory and
-// written to the wavelet plane as floats (word * step / 2) when the block is done. The
-// decoding lane is a serial chain of dependent instructions, so its length in
-// instructions is its time, and the code is kept compact: the instruction cache holds it
-// (the same loops unrolled to keep whole stripes in registers ran 1.6x slower). Untrusted
-// input: bytes past the codeword read as 0xFF, a block whose bytes lie outside the
-// codestream decodes as zero, and nothing outside the block's own samples is written.
+// on SMs of their own. All lanes run the MQ decoder in step, each also holding one column of
+// the block as row masks (t1_masks.cuh): the decoder's serial chain takes one lane's time, and
+// the contexts, the refinement pass's list, the bit-planes and the dequantisation are done for
+// all columns at once. Untrusted input: bytes past the codeword read as 0xFF, a block whose
+// bytes lie outside the codestream decodes as zero, and nothing outside the block's own
+// samples is written.
 //
 // Inverse wavelet (invLevelKernel): per level, 64 x 64 output tiles with a 4-sample halo
 // in the interleaved domain, rows then columns (the reference's order), a thread per line,
@@ -38,6 +29,7 @@
 #include "common.cuh"
 #include "decoder.h"
 #include "pool.h"
+#include "t1_masks.cuh"
 #include "t1_tables.h"
 #include "tuning.h"
 
@@ -45,14 +37,13 @@ namespace gb {
 
 namespace {
 
-// One code-block per warp: its lane 0 decodes it (the decode of a block is a serial chain
-// whose control flow depends on every decoded bit, so lanes of one warp decoding different
-// blocks would run one after another anyway); up to 32 such warps per SM keep the
-// schedulers busy.
+// One code-block per warp: the decode of a block is a serial chain whose control flow depends
+// on every decoded bit, so lanes of one warp decoding different blocks would run one after
+// another.
 constexpr int DEC_THREADS = 32;
+constexpr int DEC_CTAS = 24;  // resident warps per SM the registers must allow
 constexpr int ORDER_BUCKETS = 128;
 
-__constant__ uint8_t c_zc[4 * 45];
 __constant__ uint8_t c_sc[9];
 __constant__ uint32_t c_mq[47];
 
@@ -122,14 +113,20 @@ __global__ void __launch_bounds__(1024) orderKernel(DecArgs a) {
         if (a.blocks[i].wanted) a.perm[atomicAdd(&hist[lenBucket(a.codes[i].len)], 1u)] = i;
 }
 
-// A block's first kCwCache codeword bytes are copied into shared memory before it is decoded.
+// A block's first kCwCache codeword bytes (and two 0xFF after a shorter codeword) are copied
+// into shared memory before it is decoded.
 constexpr uint32_t kCwCache = 2048;
 
-// MQ decoder (ISO/IEC 15444-1 C.3) over one codeword; bytes past its end read as 0xFF. The
-// first `cached` bytes come from the shared-memory copy, so that a byte-in on the serial chain
-// does not wait for global memory.
+// Context state word: Qe << 16 | state index << 1 | MPS. s_next[word & 127] holds the words after
+// a renormalising MPS and after an LPS.
+__device__ __forceinline__ uint32_t stateWord(uint32_t idx, uint32_t mps) { return (c_mq[idx] << 16) | (idx << 1) | mps; }
+
+// MQ decoder (ISO/IEC 15444-1 C.3) over one codeword; bytes past its end read as 0xFF. Every
+// lane of the warp holds the same state and takes the same decisions. A and C are kept with the
+// 16-bit interval in the upper half; the next two bytes are held in registers, so that a
+// byte-in does not wait for memory.
 struct MqDecoder {
-    uint32_t A, C, bp, end, cached;
+    uint32_t A, C, bp, end, cached, b0, b1;
     int CT;
     const uint8_t* in;
     const uint8_t* cache;
@@ -137,35 +134,18 @@ struct MqDecoder {
     __device__ __forceinline__ uint32_t at(uint32_t i) const {
         return i < cached ? (uint32_t)cache[i] : (i < end ? (uint32_t)in[i] : 0xFFu);
     }
-    // The decision in context state t when it is its context's MPS, 0, with no renormalisation:
-    // then only the interval changes (the context keeps its state), and it is made here; false
-    // (nothing changed) otherwise.
-    __device__ __forceinline__ bool fastZero(uint32_t t) {
-        const uint32_t qe = t & 0xFFFFu;
-        if ((t >> 16) & 1u) return false;
-        if ((C >> 16) < qe) return false;
-        const uint32_t a = A - qe;
-        if (!(a & 0x8000u)) return false;
-        A = a;
-        C -= qe << 16;
-        return true;
-    }
     __device__ __forceinline__ void bytein() {
-        const uint32_t b = at(bp), b1 = at(bp + 1);
-        if (b == 0xFFu) {
-            if (b1 > 0x8Fu) {  // a marker: not consumed, ones from here on
-                C += 0xFF00u;
-                CT = 8;
-            } else {
-                ++bp;
-                C += b1 << 9;
-                CT = 7;
-            }
-        } else {
-            ++bp;
-            C += b1 << 8;
+        const bool stuffed = b0 == 0xFFu;
+        if (stuffed && b1 > 0x8Fu) {  // a marker: not consumed, ones from here on
+            C += 0xFF00u;
             CT = 8;
+            return;
         }
+        C += b1 << (stuffed ? 9 : 8);
+        CT = stuffed ? 7 : 8;
+        ++bp;
+        b0 = b1;
+        b1 = at(bp + 1);
     }
     __device__ __forceinline__ void init(const uint8_t* data, uint32_t len, const uint8_t* copy, uint32_t copied) {
         in = data;
@@ -173,330 +153,335 @@ struct MqDecoder {
         cache = copy;
         cached = copied;
         bp = 0;
-        C = at(0) << 16;
+        b0 = at(0);
+        b1 = at(1);
+        C = b0 << 16;
         bytein();
         C <<= 7;
         CT -= 7;
-        A = 0x8000u;
+        A = 0x80000000u;
     }
-    __device__ __forceinline__ void renorm() {
-        int n = __clz(A) - 16;
-        if (n <= CT) {  // the usual case: the bits are already in C
-            A <<= n;
-            C <<= n;
-            CT -= n;
-            return;
+    // One decision in context state t: whether it is the LPS. succ: the state's successors;
+    // tn: the context's next state.
+    __device__ __forceinline__ bool decide(uint32_t t, uint2 succ, uint32_t& tn) {
+        const uint32_t qe = t & 0xFFFF0000u;
+        const uint32_t a = A - qe;
+        const bool lower = C < qe, big = a >= qe;  // conditional exchange: the LPS has the larger part
+        const bool lps = lower == big;
+        A = lower ? qe : a;
+        C -= lower ? 0u : qe;
+        tn = (int)A >= 0 ? (lps ? succ.y : succ.x) : t;  // a renormalisation moves the state
+        int n = __clz((int)A);
+        A <<= n;
+        if (n > CT) {  // the bits are not in C yet
+            do {
+                C <<= CT;
+                n -= CT;
+                bytein();
+            } while (n > CT);
         }
-        do {
-            if (CT == 0) bytein();
-            const int s = min(n, CT);
-            A <<= s;
-            C <<= s;
-            CT -= s;
-            n -= s;
-        } while (n > 0);
-    }
-    // One decision in the context whose state word t a register holds (updated in place).
-    __device__ __forceinline__ uint32_t decodeIn(uint32_t& t, const uint32_t* tab) {
-        const uint32_t qe = t & 0xFFFFu, mps = (t >> 16) & 1u;
-        A -= qe;
-        bool lps;
-        if ((C >> 16) < qe) {
-            lps = A >= qe;
-            A = qe;
-        } else {
-            C -= qe << 16;
-            if (A & 0x8000u) return mps;
-            lps = A < qe;
-        }
-        const uint32_t nidx = lps ? (t >> 24) & 63u : (t >> 18) & 63u;
-        const uint32_t nm = mps ^ (lps ? (t >> 17) & 1u : 0u);
-        t = tab[nidx] | (nm << 16);
-        renorm();
-        return lps ? mps ^ 1u : mps;
-    }
-    // One decision in context cx (state word: table entry | mps << 16).
-    __device__ __forceinline__ uint32_t decode(uint32_t* ctx, int cx, const uint32_t* tab) {
-        uint32_t t = ctx[cx];
-        const uint32_t qe = t & 0xFFFFu, mps = (t >> 16) & 1u;
-        A -= qe;
-        bool lps;
-        if ((C >> 16) < qe) {
-            lps = A >= qe;  // conditional exchange in the lower sub-interval
-            A = qe;
-        } else {
-            C -= qe << 16;
-            if (A & 0x8000u) return mps;
-            lps = A < qe;
-        }
-        const uint32_t nidx = lps ? (t >> 24) & 63u : (t >> 18) & 63u;
-        const uint32_t nm = mps ^ (lps ? (t >> 17) & 1u : 0u);
-        ctx[cx] = tab[nidx] | (nm << 16);
-        renorm();
-        return lps ? mps ^ 1u : mps;
+        C <<= n;
+        CT -= n;
+        return lps;
     }
 };
 
-__device__ __forceinline__ uint32_t bt(uint32_t m, int x) { return (m >> x) & 1u; }
-// Row bits x-1, x, x+1 of a 32-column row mask at bits 0..2 (zero outside the block).
-__device__ __forceinline__ uint32_t win3(uint32_t row, int x) { return __funnelshift_r(row << 1, row >> 31, x) & 7u; }
-// Neighbour key of sample (x, row M) from the rows above (U) and below (D): bits 0-2 row
-// above columns x-1..x+1, 3 and 5 same row columns x-1 and x+1, 6-8 row below.
-__device__ __forceinline__ uint32_t nbKey(uint32_t U, uint32_t M, uint32_t D, int x) {
-    return win3(U, x) | ((win3(M, x) & 5u) << 3) | (win3(D, x) << 6);
-}
-
-struct BlockCtx {
-    uint32_t* sig;  // significance rows -1..32 at index y + 1
-    uint32_t* sgn;  // sign rows, the same indexing
-    uint32_t* words;  // the block's decoded words, 32 per row (shared memory)
-    const uint8_t* zk;  // zero-coding context by neighbour key, this block's orientation
-    const uint8_t* sk;  // sign context | xor bit << 5 by the sign key
-    const uint32_t* tab;
-    uint32_t* ctx;
+// One code-block by one warp. Bound by the MQ decoder's serial chain: a frame's time is at
+// least its longest block's. All lanes run the decoder in step, each lane also holding one
+// column of the block as row masks and (lanes 0-18) one context's state, so that everything but
+// the chain is done for all columns at once: the contexts of a stripe come from boolean
+// operations on whole columns, a sample's from one shuffle, a context's state from another.
+// The refinement pass changes no significance, so its contexts are laid out as a list first
+// and the chain runs down the list with its three states in registers; the bits are put back
+// into the columns afterwards. On a B200, the Tier-1 of a 4K picture at 250 Mbit/s: 1.75 ms,
+// where lane 0 alone, a sample at a time with the state in shared memory, took 2.39. (The
+// longest block spends 188 cycles per refinement decision, about 400 per other one. Slower:
+// code bytes fed ahead of their time to save the byte-in's branch, 2.3 ms; flag words per column
+// and stripe in shared memory for the contexts, 2.2 ms.)
+struct BlockDecoder {
+    uint32_t sig, sgn, vis, refined, plane;  // this lane's column; plane: the bits of the plane in hand
+    uint32_t state;                          // lanes 0-18: the context's state word
+    uint32_t left, right;                    // the neighbouring columns' significance
+    const uint2* next;
+    const uint8_t* sk;
     MqDecoder mq;
+    int lane, orient;
 
-    // Sample (x, y) with significance rows U, M, D (y - 1, y, y + 1) has its first 1-bit
-    // in plane p: decode its sign, set its significance (M too) and write sign, bit and
-    // mid-point.
-    __device__ __forceinline__ void becomeSig(uint32_t U, uint32_t& M, uint32_t D, int x, int y, int p) {
-        const uint32_t GU = sgn[y], GM = sgn[y + 1], GD = sgn[y + 2];
-        const uint32_t key = (win3(M, x) & 5u) | ((win3(GM, x) & 5u) << 1) | (bt(U, x) << 4) | (bt(GU, x) << 5) |
-                             (bt(D, x) << 6) | (bt(GD, x) << 7);
+    // One decision in context cx.
+    __device__ __forceinline__ uint32_t decode(uint32_t cx) {
+        const uint32_t t = __shfl_sync(kFull, state, (int)cx);
+        uint32_t tn;
+        const bool lps = mq.decide(t, next[t & 127u], tn);
+        if ((uint32_t)lane == cx) state = tn;
+        return (t & 1u) ^ (lps ? 1u : 0u);
+    }
+    // The stripe at row r0 as the scan now stands: zc = the zero-coding contexts of its four
+    // rows in this lane's column, a byte each (0: no significant neighbour); returns the rows
+    // with a significant neighbour.
+    __device__ __forceinline__ uint32_t contexts(int r0, uint32_t& zc) {
+        left = shUp(sig, lane);
+        right = shDown(sig, lane);
+        Nbr q;
+        q.l = left;
+        q.lu = left << 1;
+        q.ld = left >> 1;
+        q.r = right;
+        q.ru = right << 1;
+        q.rd = right >> 1;
+        q.u = sig << 1;
+        q.d = sig >> 1;
+        uint32_t c0, c1, c2, c3;
+        zcMasks(q, orient, c0, c1, c2, c3);
+        zc = spread1((c0 >> r0) & 0xFu) | (spread1((c1 >> r0) & 0xFu) << 1) | (spread1((c2 >> r0) & 0xFu) << 2) |
+             (spread1((c3 >> r0) & 0xFu) << 3);
+        return q.l | q.lu | q.ld | q.r | q.ru | q.rd | q.u | q.d;
+    }
+    // Sample (x, r) has its first 1-bit in this plane: its sign, and its significance.
+    __device__ __forceinline__ void becomeSig(int x, int r) {
+        const uint32_t gl = shUp(sgn, lane), gr = shDown(sgn, lane);
+        uint32_t key = ((left >> r) & 1u) | (((gl >> r) & 1u) << 1) | (((right >> r) & 1u) << 2) | (((gr >> r) & 1u) << 3) |
+                       ((((sig << 1) >> r) & 1u) << 4) | ((((sgn << 1) >> r) & 1u) << 5) |
+                       ((((sig >> 1) >> r) & 1u) << 6) | ((((sgn >> 1) >> r) & 1u) << 7);
+        key = __shfl_sync(kFull, key, x);
         const uint32_t c = sk[key];
-        const uint32_t neg = mq.decode(ctx, c & 31u, tab) ^ (c >> 5);
-        M |= 1u << x;
-        sig[y + 1] = M;
-        sgn[y + 1] = GM | (neg << x);
-        words[y * 32 + x] = (neg << 31) | (3u << p);
+        const uint32_t neg = decode(c & 31u) ^ (c >> 5);
+        if (lane == x) {
+            sig |= 1u << r;
+            plane |= 1u << r;
+            sgn |= neg << r;
+        }
     }
 };
 
-__global__ void __launch_bounds__(DEC_THREADS) decodeKernel(DecArgs a) {
-    // per block: significance and sign of rows -1..32, coded-this-plane and refined rows 0..31
-    __shared__ uint32_t s_sig[34], s_sgn[34], s_vis[32], s_ref[32];
-    // the block's decoded words (sign, twice the magnitude plus the mid-point of the planes
-    // not decoded), kept here and turned into floats in the plane when the block is done:
-    // each refinement updates its word, and a global read-modify-write per refinement put a
-    // memory round trip on the decoder's serial chain. Only significant samples' words are
-    // ever read, and each is written when its sample becomes significant.
-    __shared__ uint32_t s_word[32 * 32];
-    __shared__ uint32_t s_ctx[19];
-    __shared__ uint32_t s_tab[48];
-    __shared__ uint8_t s_cw[kCwCache];  // the block's codeword, its first kCwCache bytes
-    __shared__ uint8_t s_zc[4 * 45], s_sc[16];
-    // zero coding by orientation and neighbour key (nbKey); sign coding by the sign key:
-    // bits 0/1 left neighbour significant/negative, 2/3 right, 4/5 above, 6/7 below
-    __shared__ uint8_t s_zk[4 * 512], s_sk[256];
-    for (int i = threadIdx.x; i < 47; i += blockDim.x) s_tab[i] = c_mq[i];
-    for (int i = threadIdx.x; i < 4 * 45; i += blockDim.x) s_zc[i] = c_zc[i];
-    if (threadIdx.x < 9) s_sc[threadIdx.x] = c_sc[threadIdx.x];
-    __syncthreads();
-    for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) {
-        const int o = i >> 9, k = i & 511;
-        const int h = ((k >> 3) & 1) + ((k >> 5) & 1);
-        const int v = ((k >> 1) & 1) + ((k >> 7) & 1);
-        const int d = (k & 1) + ((k >> 2) & 1) + ((k >> 6) & 1) + ((k >> 8) & 1);
-        s_zk[i] = s_zc[45 * o + h + 3 * v + 9 * d];
+__global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decodeKernel(DecArgs a) {
+    // the block's decoded bit-planes, a column per lane
+    __shared__ uint32_t s_plane[30][32];
+    __shared__ uint32_t s_list[kCblkArea / 4 + 2];  // a refinement pass's contexts, a byte each
+    __shared__ uint32_t s_bits[kCblkArea / 32 + 2];  // and its decoded bits
+    __shared__ uint2 s_next[2 * 47];
+    __shared__ uint8_t s_cw[kCwCache + 2];  // the block's codeword, its first kCwCache bytes
+    // sign coding, context | xor bit << 5, by the sign key: bits 0/1 left neighbour
+    // significant/negative, 2/3 right, 4/5 above, 6/7 below
+    __shared__ uint8_t s_sk[256];
+    const int lane = threadIdx.x;
+    for (int i = lane; i < 2 * 47; i += 32) {
+        const uint32_t e = c_mq[i >> 1], mps = i & 1u;
+        s_next[i] = make_uint2(stateWord((e >> 18) & 63u, mps), stateWord((e >> 24) & 63u, mps ^ ((e >> 17) & 1u)));
     }
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) {
+    for (int k = lane; k < 256; k += 32) {
         auto chi = [&](int bit) { return ((k >> bit) & 1) ? (((k >> (bit + 1)) & 1) ? -1 : 1) : 0; };
         const int hc = max(-1, min(1, chi(0) + chi(2)));
         const int vc = max(-1, min(1, chi(4) + chi(6)));
-        s_sk[k] = s_sc[(hc + 1) * 3 + (vc + 1)];
+        s_sk[k] = c_sc[(hc + 1) * 3 + (vc + 1)];
     }
-    __syncthreads();
-    const uint32_t lane = threadIdx.x;
-    BlockCtx b;
-    b.sig = s_sig;
-    b.sgn = s_sgn;
-    b.sk = s_sk;
-    b.tab = s_tab;
-    b.ctx = s_ctx;
+    __syncwarp();
+    BlockDecoder d;
+    d.next = s_next;
+    d.sk = s_sk;
+    d.lane = lane;
     const uint32_t count = a.ctl[2], heavy = a.ctl[3];
-    auto decodeBlock = [&](uint32_t j) {
-        const DecBlock blk = a.blocks[j];
-        const GbCblkCode code = a.codes[j];
-        const int w = blk.w, h = blk.h;
-        uint32_t* out = a.planes + blk.dst;  // zeroed before the launch: only significant samples are written
-        const int nbps = code.nbps;
-        const bool valid = code.passes > 0 && nbps >= 1 && nbps <= 30 && (uint64_t)code.offset + code.len <= a.size;
-        if (!valid) return;
-        b.words = s_word;
-        b.zk = s_zk + 512 * blk.orient;
-        for (int i = 0; i < 34; ++i) s_sig[i] = s_sgn[i] = 0;
-        for (int i = 0; i < 32; ++i) s_vis[i] = s_ref[i] = 0;
-        for (int c = 0; c < 19; ++c) s_ctx[c] = s_tab[0];
-        s_ctx[0] = s_tab[4];
-        s_ctx[17] = s_tab[3];
-        s_ctx[18] = s_tab[46];
-        b.mq.init(a.bytes + code.offset, code.len, s_cw, min(code.len, kCwCache));
-        const uint32_t wmask = w >= 32 ? 0xFFFFFFFFu : (1u << w) - 1u;
-        int done = 0;
-        const int passes = code.passes;
-        for (int p = nbps - 1; p >= 0 && done < passes; --p) {
-            for (int type = (p == nbps - 1 ? 2 : 0); type < 3 && done < passes; ++type, ++done) {
-                // the refinement pass keeps its three contexts (14-16) in registers
-                uint32_t t14 = 0, t15 = 0, t16 = 0;
-                if (type == 1) {
-                    t14 = s_ctx[14];
-                    t15 = s_ctx[15];
-                    t16 = s_ctx[16];
+
+    auto decodeBlock = [&](const DecBlock& blk, const GbCblkCode& code) {
+        const int w = blk.w, h = blk.h, nbps = code.nbps;
+        const uint32_t valid = lane < w ? (h >= 32 ? kFull : (1u << h) - 1u) : 0u;
+        d.orient = blk.orient;
+        d.sig = d.sgn = d.refined = 0;
+        // initial states, Table D.7: ZC context 0 state 4, run-length 3, uniform 46
+        d.state = stateWord(lane == 0 ? 4u : lane == 17 ? 3u : lane == 18 ? 46u : 0u, 0u);
+        d.mq.init(a.bytes + code.offset, code.len, s_cw, min(code.len, kCwCache) + 2u);
+        int passes = code.passes, p = nbps;
+        uint32_t coded = 0;  // samples coded in the plane in hand
+        while (passes > 0 && p > 0) {
+            --p;
+            const uint32_t sig0 = d.sig;
+            d.vis = d.plane = coded = 0;
+            if (p != nbps - 1) {
+                // significance propagation
+                for (int r0 = 0; r0 < h; r0 += 4) {
+                    uint32_t zc;
+                    uint32_t e4 = ((d.contexts(r0, zc) & valid & ~d.sig) >> r0) & 0xFu;
+                    uint32_t cols = __ballot_sync(kFull, e4 != 0);
+                    while (cols) {
+                        const int x = __ffs(cols) - 1;
+                        cols &= cols - 1;
+                        uint32_t e = __shfl_sync(kFull, e4, x), z = __shfl_sync(kFull, zc, x), seen = 0;
+                        while (e) {
+                            const int i = __ffs(e) - 1;
+                            e &= e - 1;
+                            seen |= 1u << i;
+                            if (!d.decode((z >> (8 * i)) & 0xFFu)) continue;
+                            d.becomeSig(x, r0 + i);
+                            // what the scan has not passed may now be eligible
+                            e4 = ((d.contexts(r0, zc) & valid & ~d.sig) >> r0) & 0xFu;
+                            z = __shfl_sync(kFull, zc, x);
+                            e = __shfl_sync(kFull, e4, x) & ~((2u << i) - 1u);
+                            cols = __ballot_sync(kFull, e4 != 0) & ~((2u << x) - 1u);
+                        }
+                        if (lane == x) d.vis |= seen << r0;
+                    }
                 }
-                // stripes of four rows from y0; rows y0-1..y0+4 lie in -1..32 (y0 <= 28) and
-                // rows at or past h are zero. Each column is scanned top to bottom with the
-                // rows above, at and below the sample in U, M, D.
-                for (int y0 = 0; y0 < h; y0 += 4) {
-                    const int n = min(4, h - y0);
-                    if (type == 0) {  // significance propagation
-                        uint32_t cm = 0;
-                        for (int k = 0; k < n; ++k) {
-                            const uint32_t U = s_sig[y0 + k], M = s_sig[y0 + k + 1], D = s_sig[y0 + k + 2];
-                            cm |= (U | (U << 1) | (U >> 1) | (M << 1) | (M >> 1) | D | (D << 1) | (D >> 1)) & ~M;
-                        }
-                        cm &= wmask;
-                        while (cm) {
-                            const int x = __ffs(cm) - 1;
-                            cm &= cm - 1;
-                            uint32_t U = s_sig[y0], M = s_sig[y0 + 1];
-                            for (int k = 0; k < n; ++k) {
-                                const int y = y0 + k;
-                                const uint32_t D = s_sig[y + 2];
-                                if (!bt(M, x)) {
-                                    const uint32_t key = nbKey(U, M, D, x);
-                                    if (key) {
-                                        const uint32_t bit = b.mq.decode(s_ctx, b.zk[key], s_tab);
-                                        s_vis[y] |= 1u << x;
-                                        if (bit) {
-                                            b.becomeSig(U, M, D, x, y, p);
-                                            cm |= (2u << x) & wmask;  // the next column may now be eligible
-                                        }
-                                    }
-                                }
-                                U = M;
-                                M = D;
-                            }
-                        }
-                    } else if (type == 1) {  // magnitude refinement
-                        // nothing changes significance in this pass, so every sample's context
-                        // is known before it: per row of the stripe, the samples to refine
-                        // (significant before this plane, not coded in it), those refined
-                        // before (context 16) and those with a significant neighbour (15,
-                        // else 14); per column their four rows as nibbles
-                        uint32_t e4[4] = {0, 0, 0, 0}, r4[4] = {0, 0, 0, 0}, n4[4] = {0, 0, 0, 0};
-                        uint32_t cm = 0;
+                coded = d.vis;
+                if (--passes > 0) {
+                    // magnitude refinement: the list of the pass's contexts (2: refined before, 1: a
+                    // significant neighbour, 0), stripe by stripe, column by column
+                    const uint32_t E = sig0;
+                    d.left = shUp(d.sig, lane);
+                    d.right = shDown(d.sig, lane);
+                    const uint32_t nAny = (d.sig << 1) | (d.sig >> 1) | d.left | (d.left << 1) | (d.left >> 1) | d.right |
+                                          (d.right << 1) | (d.right >> 1);
+                    uint32_t m[8] = {nAny & ~d.refined, d.refined, 0u, 0u, 0u, 0u, 0u, 0u};
+                    rowBytes(m);
+                    const uint32_t c = nibbleCounts(E);
+                    const uint32_t w0 = (c & 0xFu) | (((c >> 4) & 0xFu) << 10) | (((c >> 8) & 0xFu) << 20);
+                    const uint32_t w1 = ((c >> 12) & 0xFu) | (((c >> 16) & 0xFu) << 10) | (((c >> 20) & 0xFu) << 20);
+                    const uint32_t w2 = ((c >> 24) & 0xFu) | ((c >> 28) << 10);
+                    const uint32_t i0 = warpScan(w0, lane), i1 = warpScan(w1, lane), i2 = warpScan(w2, lane);
+                    const uint32_t x0 = i0 - w0, x1 = i1 - w1, x2 = i2 - w2;
+                    const uint32_t t0 = __shfl_sync(kFull, i0, 31), t1 = __shfl_sync(kFull, i1, 31),
+                                   t2 = __shfl_sync(kFull, i2, 31);
+                    uint32_t total = 0;
+                    uint8_t* list = reinterpret_cast<uint8_t*>(s_list);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            if (k >= n) break;
-                            const uint32_t U = s_sig[y0 + k], M = s_sig[y0 + k + 1], D = s_sig[y0 + k + 2];
-                            e4[k] = M & ~s_vis[y0 + k];
-                            r4[k] = s_ref[y0 + k];
-                            n4[k] = U | (U << 1) | (U >> 1) | (M << 1) | (M >> 1) | D | (D << 1) | (D >> 1);
-                            cm |= e4[k];
-                        }
-                        while (cm) {
-                            const int x = __ffs(cm) - 1;
-                            cm &= cm - 1;
-                            const uint32_t ec = bt(e4[0], x) | bt(e4[1], x) << 1 | bt(e4[2], x) << 2 | bt(e4[3], x) << 3;
-                            const uint32_t rc = bt(r4[0], x) | bt(r4[1], x) << 1 | bt(r4[2], x) << 2 | bt(r4[3], x) << 3;
-                            const uint32_t nc = bt(n4[0], x) | bt(n4[1], x) << 1 | bt(n4[2], x) << 2 | bt(n4[3], x) << 3;
-                            for (uint32_t m = ec; m; m &= m - 1) {
-                                const int k = __ffs(m) - 1;
-                                const bool c16 = bt(rc, k), c15 = bt(nc, k);
-                                uint32_t t = c16 ? t16 : (c15 ? t15 : t14);
-                                const uint32_t bit = b.mq.decodeIn(t, s_tab);
-                                if (c16) t16 = t;
-                                else if (c15) t15 = t;
-                                else t14 = t;
-                                uint32_t& word = s_word[(y0 + k) * 32 + x];
-                                word = bit ? word + (1u << p) : word - (1u << p);
-                            }
-                        }
-                        // every sample refined here counts as refined from now on
+                    for (int s = 0; s < 8; ++s) {
+                        const int sh = 10 * (s % 3);
+                        uint8_t* o = list + total + (((s < 3 ? x0 : (s < 6 ? x1 : x2)) >> sh) & 1023u);
+                        total += ((s < 3 ? t0 : (s < 6 ? t1 : t2)) >> sh) & 1023u;
+                        uint32_t z = m[s];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k < n) s_ref[y0 + k] = r4[k] | e4[k];
-                    } else {  // cleanup, with run-length coding of quiet columns
-                        uint32_t cm = 0, any = s_sig[y0], vis = 0;
-                        for (int k = 0; k < n; ++k) {
-                            const uint32_t M = s_sig[y0 + k + 1], V = s_vis[y0 + k];
-                            cm |= ~M & ~V;
-                            any |= M;
-                            vis |= V;
+                        for (int i = 0; i < 4; ++i, z >>= 8)
+                            if (E & (1u << (4 * s + i))) *o++ = (uint8_t)z;
+                    }
+                    __syncwarp();
+                    // the chain, its three states in registers
+                    uint32_t s14 = __shfl_sync(kFull, d.state, 14), s15 = __shfl_sync(kFull, d.state, 15),
+                             s16 = __shfl_sync(kFull, d.state, 16);
+                    auto refine = [&](uint32_t cx) {
+                        const uint32_t t = cx == 2u ? s16 : (cx == 1u ? s15 : s14);
+                        uint32_t tn;
+                        const bool lps = d.mq.decide(t, s_next[t & 127u], tn);
+                        s16 = cx == 2u ? tn : s16;
+                        s15 = cx == 1u ? tn : s15;
+                        s14 = cx == 0u ? tn : s14;
+                        return (t & 1u) ^ (lps ? 1u : 0u);
+                    };
+                    uint32_t acc = 0, codes = s_list[0];
+                    const uint32_t whole = total & ~3u;
+#pragma unroll 1
+                    for (uint32_t k = 0; k < whole; k += 4) {
+                        const uint32_t ahead = s_list[(k >> 2) + 1];
+                        uint32_t four = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) four |= refine((codes >> (8 * i)) & 3u) << i;
+                        acc |= four << (k & 31u);
+                        if ((k & 31u) == 28u) {
+                            if (lane == 0) s_bits[k >> 5] = acc;
+                            acc = 0;
                         }
-                        any |= s_sig[y0 + n + 1];
-                        cm &= wmask;
-                        while (cm) {
-                            int x = __ffs(cm) - 1;
-                            if (n == 4) {
-                                // quiet columns whose run-length decision is a 0 that is its
-                                // context's MPS and needs no renormalisation: nothing in them,
-                                // and only the interval changes
-                                const uint32_t t17 = s_ctx[17];
-                                while (!win3(any, x) && !bt(vis, x) && b.mq.fastZero(t17)) {
-                                    cm &= cm - 1;
-                                    if (!cm) break;
-                                    x = __ffs(cm) - 1;
-                                }
-                                if (!cm) break;
+                        codes = ahead;
+                    }
+#pragma unroll 1
+                    for (uint32_t k = whole; k < total; ++k, codes >>= 8) acc |= refine(codes & 3u) << (k & 31u);
+                    if (lane == 0) s_bits[total >> 5] = acc;
+                    if (lane == 14) d.state = s14;
+                    if (lane == 15) d.state = s15;
+                    if (lane == 16) d.state = s16;
+                    __syncwarp();
+                    total = 0;
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        const int sh = 10 * (s % 3);
+                        const uint32_t at = total + (((s < 3 ? x0 : (s < 6 ? x1 : x2)) >> sh) & 1023u);
+                        total += ((s < 3 ? t0 : (s < 6 ? t1 : t2)) >> sh) & 1023u;
+                        uint32_t bits = __funnelshift_r(s_bits[at >> 5], s_bits[(at >> 5) + 1], at & 31u);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (E & (1u << (4 * s + i))) {
+                                d.plane |= (bits & 1u) << (4 * s + i);
+                                bits >>= 1;
                             }
-                            cm &= cm - 1;
-                            int r = 0;
-                            // quiet column: nothing significant in rows y0-1..y0+4 around it and
-                            // nothing coded in this plane in it
-                            if (n == 4 && !win3(any, x) && !bt(vis, x)) {
-                                if (!b.mq.decode(s_ctx, 17, s_tab)) continue;
-                                int first = (int)b.mq.decode(s_ctx, 18, s_tab) << 1;
-                                first |= (int)b.mq.decode(s_ctx, 18, s_tab);
-                                uint32_t M = s_sig[y0 + first + 1];
-                                b.becomeSig(s_sig[y0 + first], M, s_sig[y0 + first + 2], x, y0 + first, p);
-                                any |= 1u << x;
-                                r = first + 1;
+                    }
+                    __syncwarp();
+                    d.refined |= E;
+                    coded |= E;
+                    --passes;
+                }
+            }
+            if (passes > 0) {
+                // cleanup, with run-length coding of quiet columns
+                const uint32_t E = valid & ~d.sig & ~d.vis;
+                for (int r0 = 0; r0 < h; r0 += 4) {
+                    const uint32_t e4 = (E >> r0) & 0xFu;
+                    uint32_t cols = __ballot_sync(kFull, e4 != 0);
+                    if (!cols) continue;
+                    uint32_t zc;
+                    d.contexts(r0, zc);
+                    // quiet columns: all four rows in cleanup, none with a significant neighbour
+                    uint32_t runs = __ballot_sync(kFull, e4 == 0xFu && zc == 0u);
+                    while (cols) {
+                        const int x = __ffs(cols) - 1;
+                        cols &= cols - 1;
+                        uint32_t e = __shfl_sync(kFull, e4, x), z = __shfl_sync(kFull, zc, x);
+                        int i = -1;  // the row that turned significant
+                        if ((runs >> x) & 1u) {
+                            if (!d.decode(17u)) continue;
+                            i = (int)d.decode(18u) << 1;
+                            i |= (int)d.decode(18u);
+                        }
+                        for (;;) {
+                            if (i >= 0) {
+                                d.becomeSig(x, r0 + i);
+                                d.contexts(r0, zc);
+                                z = __shfl_sync(kFull, zc, x);
+                                e &= ~((2u << i) - 1u);
+                                runs = __ballot_sync(kFull, e4 == 0xFu && zc == 0u);
                             }
-                            uint32_t U = s_sig[y0 + r], M = s_sig[y0 + r + 1];
-                            for (int k = r; k < n; ++k) {
-                                const int y = y0 + k;
-                                const uint32_t D = s_sig[y + 2];
-                                if (!bt(M | s_vis[y], x)) {
-                                    const uint32_t bit = b.mq.decode(s_ctx, b.zk[nbKey(U, M, D, x)], s_tab);
-                                    if (bit) {
-                                        b.becomeSig(U, M, D, x, y, p);
-                                        any |= 1u << x;
-                                    }
-                                }
-                                U = M;
-                                M = D;
+                            i = -1;
+                            while (e && i < 0) {
+                                const int k = __ffs(e) - 1;
+                                e &= e - 1;
+                                if (d.decode((z >> (8 * k)) & 0xFFu)) i = k;
                             }
+                            if (i < 0) break;
                         }
                     }
                 }
-                if (type == 1) {
-                    s_ctx[14] = t14;
-                    s_ctx[15] = t15;
-                    s_ctx[16] = t16;
-                }
+                coded |= E;
+                --passes;
             }
-            for (int i = 0; i < 32; ++i) s_vis[i] = 0;
+            s_plane[p][lane] = d.plane;  // read by this lane alone
         }
-        // dequantise into the plane, the significant samples only (every other sample
-        // is 0, which is 0.0f): word * step / 2, sign from bit 31
-        const float half = a.half[blk.band];
-        float* f = reinterpret_cast<float*>(out);
-        for (int y = 0; y < h; ++y)
-            for (uint32_t m = s_sig[y + 1] & wmask; m; m &= m - 1) {
-                const int x = __ffs(m) - 1;
-                const uint32_t v = s_word[y * 32 + x];
-                const float mag = (float)(v & 0x7FFFFFFFu) * half;
-                f[(size_t)y * a.W + x] = (v & 0x80000000u) ? -mag : mag;
+        // The words of the column: the sign, twice the magnitude, and the mid-point of the planes
+        // not decoded (below the last plane for the samples coded in it, else one above), then
+        // rows: a transpose, and word * step / 2 in floats.
+        uint32_t v[32];
+#pragma unroll
+        for (int k = 0; k < 30; ++k) v[k + 1] = k >= p && k < nbps ? s_plane[k][lane] : 0u;
+        v[0] = 0u;
+        v[31] = d.sgn;
+#pragma unroll
+        for (int k = 0; k < 30; ++k)
+            if (k == p) {
+                v[k] |= d.sig & coded;
+                v[k + 1] |= d.sig & ~coded;
             }
+        transpose32(v);
+        const float half = a.half[blk.band];
+        float* out = reinterpret_cast<float*>(a.planes + blk.dst) + lane;
+        if (lane < w) {
+#pragma unroll
+            for (int r = 0; r < 32; ++r)
+                if (r < h) {
+                    const float mag = (float)(v[r] & 0x7FFFFFFFu) * half;
+                    out[(size_t)r * a.W] = (v[r] & 0x80000000u) ? -mag : mag;
+                }
+        }
     };
 
-    // Every lane stays: lane 0 picks each block and decodes it, the others first copy its
-    // codeword into shared memory with it. The heavy blocks (the first of the order): on a
-    // reserved SM (%smid below the reserved count), the first four warps to arrive take one
-    // each and every other warp leaves, so that the SM runs their serial chains alone; the
-    // other warps take blocks from the queue, then any heavy block no reserved SM's warp took
-    // (a grid that did not reach every reserved SM).
+    // Lane 0 picks each block. The heavy blocks (the first of the order): on a reserved SM
+    // (%smid below the reserved count), the first four warps to arrive take one each and every
+    // other warp leaves, so that the SM runs their serial chains alone; the other warps take
+    // blocks from the queue, then any heavy block no reserved SM's warp took (a grid that did
+    // not reach every reserved SM).
     uint32_t smid;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     const uint32_t reserved = (heavy + 3) / 4;
@@ -522,13 +507,22 @@ __global__ void __launch_bounds__(DEC_THREADS) decodeKernel(DecArgs a) {
         }
         j = __shfl_sync(kFull, j, 0);
         if (j == 0xFFFFFFFFu) break;
-        const GbCblkCode code = a.codes[j];
-        if ((uint64_t)code.offset + code.len <= a.size) {
-            const uint8_t* src = a.bytes + code.offset;
-            for (uint32_t i = lane; i < min(code.len, kCwCache); i += 32) s_cw[i] = src[i];
+        const DecBlock blk = a.blocks[j];
+        GbCblkCode code = a.codes[j];
+        // a block that cannot be decoded counts as empty: all zero
+        if (code.nbps < 1 || code.nbps > 30 || (uint64_t)code.offset + code.len > a.size) code.passes = 0;
+        if (code.passes == 0) {
+            float* out = reinterpret_cast<float*>(a.planes + blk.dst) + lane;
+            if (lane < blk.w)
+                for (int r = 0; r < blk.h; ++r) out[(size_t)r * a.W] = 0.f;
+            continue;
         }
+        const uint8_t* src = a.bytes + code.offset;
+        const uint32_t kept = min(code.len, kCwCache);
+        for (uint32_t i = lane; i < kept; i += 32) s_cw[i] = src[i];
+        if (lane < 2) s_cw[kept + lane] = code.len > kept + lane ? src[kept + lane] : 0xFFu;
         __syncwarp();
-        if (lane == 0) decodeBlock(j);
+        decodeBlock(blk, code);
         __syncwarp();
     }
 }
@@ -702,7 +696,6 @@ void decoderInit() {
     uint8_t zc[4 * 45], sc[9];
     uint32_t mq[47];
     t1BuildTables(zc, sc, mq);
-    GB_CHECK(cudaMemcpyToSymbol(c_zc, zc, sizeof zc));
     GB_CHECK(cudaMemcpyToSymbol(c_sc, sc, sizeof sc));
     GB_CHECK(cudaMemcpyToSymbol(c_mq, mq, sizeof mq));
     GB_CHECK(cudaFuncSetAttribute(invLevelKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmemLast));
@@ -863,7 +856,8 @@ void DecoderSlot::enqueue(const Layout& frame, const uint8_t* data, size_t size,
     GB_CHECK(cudaMemcpyAsync(dCodes_, hCodes_, n * sizeof(GbCblkCode), cudaMemcpyHostToDevice, st));
     GB_CHECK(cudaMemcpyAsync(dHalf_, hHalf_, frame.bands.size() * 4, cudaMemcpyHostToDevice, st));
     GB_CHECK(cudaMemsetAsync(dCtl_, 0, kCtlWords * 4, st));
-    GB_CHECK(cudaMemsetAsync(dPlanes_, 0, npix * 12, st));  // coefficients of uncoded samples
+    // every sample of a wanted block is written; the tap also shows the resolutions left out
+    if (wantWavelet) GB_CHECK(cudaMemsetAsync(dPlanes_, 0, npix * 12, st));
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_);
     const Tuning tu = tuningFor(L_.profile);
