@@ -460,7 +460,7 @@ def run_ours(args):
         # codewords; packing moves the codewords and the per-block and per-pass tables
         alg = {"front": npix * 60, "cm": ncblk * 4096 + dec, "mq": dec + cod, "pack": 2 * cod + ncblk * 40}
         names = {"front": "front end (colour + 9/7 + quantisation; one CUDA graph per frame)",
-                 "cm": "Tier-1 context modelling (t1CmKernel, batched)", "order": "Tier-1 ordering (t1OrderKernel)",
+                 "cm": "Tier-1 context modelling (t1CmKernel, batched)", "order": "Tier-1 ordering (t1OrderCountKernel, t1OrderScatterKernel)",
                  "mq": "Tier-1 MQ coding + truncation lengths (t1MqKernel, t1TruncKernel)",
                  "pack": "packing + PCRD hull points (tileSum, scan, hull, copy)",
                  "rc": "rate control + Tier-2 on the device (host wall time of the round trips, per frame)"}

@@ -2,7 +2,7 @@
 // ICT and 12-bit packing.
 //
 // Tier-1 (decodeKernel): one code-block per warp at a time; up to 24 such warps per SM pull
-// blocks from a device queue ordered longest codeword first (orderKernel), the heaviest
+// blocks from a device queue ordered longest codeword first (orderScatterKernel), the heaviest
 // on SMs of their own. All lanes run the MQ decoder in step, each also holding one column of
 // the block as row masks (t1_masks.cuh): the decoder's serial chain takes one lane's time, and
 // the contexts, the refinement pass's list, the bit-planes and the dequantisation are done for
@@ -52,11 +52,13 @@ __constant__ uint32_t c_mq[47];
 // bytes or more takes the whole launch's time.
 constexpr uint32_t kMaxReserveSms = 32;
 constexpr uint32_t kMaxHeavy = 4 * kMaxReserveSms;
-// Control words: [0] queue head, [1] status, [2] wanted blocks, [3] heavy blocks, [4] the
-// wanted blocks' codeword bytes; from kCtlArrive a counter per reserved SM, from kCtlClaim a
-// claim flag per heavy block.
+// Control words: [0] queue head, [1] status, [2] wanted blocks, [3] blocks above the heavy
+// limit, [4] the wanted blocks' codeword bytes; from kCtlArrive a counter per reserved SM, from
+// kCtlClaim a claim flag per heavy block, from kCtlHist the order's bucket counts, from
+// kCtlCursor the places taken in them.
 constexpr uint32_t kCtlArrive = 16, kCtlClaim = kCtlArrive + kMaxReserveSms;
-constexpr uint32_t kCtlWords = kCtlClaim + kMaxHeavy;
+constexpr uint32_t kCtlHist = kCtlClaim + kMaxHeavy, kCtlCursor = kCtlHist + ORDER_BUCKETS;
+constexpr uint32_t kCtlWords = kCtlCursor + ORDER_BUCKETS;
 
 struct DecArgs {
     const uint8_t* bytes;
@@ -79,13 +81,16 @@ __device__ __forceinline__ uint32_t lenBucket(uint32_t len) {
     return ORDER_BUCKETS - 1 - min(4 * l + ((len >> (l - 2)) & 3u), (uint32_t)ORDER_BUCKETS - 1);
 }
 
-__global__ void __launch_bounds__(1024) orderKernel(DecArgs a) {
-    __shared__ uint32_t hist[ORDER_BUCKETS];
-    __shared__ uint32_t total, bytes, heavy;
+// The order, largest codeword first in log-spaced classes, over the whole GPU (a single CTA took
+// 58 us for a 4K frame's 25,986 blocks on a B200): per-CTA histograms and byte sums into the control
+// words; then every CTA scans the histogram for itself and places its blocks 256 at a time, one
+// atomic per bucket and CTA for their places.
+__global__ void __launch_bounds__(256) orderCountKernel(DecArgs a) {
+    __shared__ uint32_t hist[ORDER_BUCKETS], total, bytes;
     for (int i = threadIdx.x; i < ORDER_BUCKETS; i += blockDim.x) hist[i] = 0;
-    if (threadIdx.x == 0) total = bytes = heavy = 0;
+    if (threadIdx.x == 0) total = bytes = 0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x)
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x)
         if (a.blocks[i].wanted) {
             const uint32_t len = a.codes[i].len;
             atomicAdd(&hist[lenBucket(len)], 1u);
@@ -93,24 +98,48 @@ __global__ void __launch_bounds__(1024) orderKernel(DecArgs a) {
             atomicAdd(&bytes, min(len, 1u << 20));
         }
     __syncthreads();
-    // heavy blocks: above heavyPct % of the mean codeword bytes per decoding warp
-    const uint64_t limit = (uint64_t)bytes * a.heavyPct / (100ull * max(a.slots, 1u));
-    for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x)
-        if (a.heavyPct && a.blocks[i].wanted && a.codes[i].len > limit) atomicAdd(&heavy, 1u);
+    for (int b = threadIdx.x; b < ORDER_BUCKETS; b += blockDim.x)
+        if (hist[b]) atomicAdd(a.ctl + kCtlHist + b, hist[b]);
     if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int b = 0; b < ORDER_BUCKETS; ++b) {
-            const uint32_t c = hist[b];
-            hist[b] = run;
-            run += c;
-        }
-        a.ctl[2] = total;
-        a.ctl[4] = bytes;
+        atomicAdd(a.ctl + 2, total);
+        atomicAdd(a.ctl + 4, bytes);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) a.ctl[3] = min(heavy, kMaxHeavy);  // the first ones of the order
-    for (uint32_t i = threadIdx.x; i < a.n; i += blockDim.x)
-        if (a.blocks[i].wanted) a.perm[atomicAdd(&hist[lenBucket(a.codes[i].len)], 1u)] = i;
+}
+
+__global__ void __launch_bounds__(256) orderScatterKernel(DecArgs a) {
+    __shared__ uint32_t base[ORDER_BUCKETS], count[ORDER_BUCKETS], place[ORDER_BUCKETS];
+    const int tid = threadIdx.x;
+    if (tid < 32) {
+        uint32_t v[4], s = 0;
+        for (int k = 0; k < 4; ++k) {
+            v[k] = a.ctl[kCtlHist + 4 * tid + k];
+            s += v[k];
+        }
+        uint32_t run = warpScan(s, tid) - s;
+        for (int k = 0; k < 4; ++k) {
+            base[4 * tid + k] = run;
+            run += v[k];
+        }
+    }
+    // heavy blocks: above heavyPct % of the mean codeword bytes per decoding warp
+    const uint64_t limit = (uint64_t)a.ctl[4] * a.heavyPct / (100ull * max(a.slots, 1u));
+    for (uint32_t first = blockIdx.x * 256u; first < a.n; first += gridDim.x * 256u) {
+        const uint32_t i = first + tid;
+        if (tid < ORDER_BUCKETS) count[tid] = 0;
+        __syncthreads();
+        const bool wanted = i < a.n && a.blocks[i].wanted;
+        uint32_t b = 0, rank = 0;
+        if (wanted) {
+            const uint32_t len = a.codes[i].len;
+            b = lenBucket(len);
+            rank = atomicAdd(&count[b], 1u);
+            if (a.heavyPct && len > limit) atomicAdd(a.ctl + 3, 1u);
+        }
+        __syncthreads();
+        if (tid < ORDER_BUCKETS && count[tid]) place[tid] = base[tid] + atomicAdd(a.ctl + kCtlCursor + tid, count[tid]);
+        __syncthreads();
+        if (wanted) a.perm[place[b] + rank] = i;
+    }
 }
 
 // A block's first kCwCache codeword bytes (and two 0xFF after a shorter codeword) are copied
@@ -279,7 +308,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decodeKernel(DecArgs a)
     d.next = s_next;
     d.sk = s_sk;
     d.lane = lane;
-    const uint32_t count = a.ctl[2], heavy = a.ctl[3];
+    const uint32_t count = a.ctl[2], heavy = min(a.ctl[3], kMaxHeavy);  // the first ones of the order
 
     auto decodeBlock = [&](const DecBlock& blk, const GbCblkCode& code) {
         const int w = blk.w, h = blk.h, nbps = code.nbps;
@@ -864,7 +893,9 @@ void DecoderSlot::enqueue(const Layout& frame, const uint8_t* data, size_t size,
     const uint32_t grid = std::min<uint32_t>((uint32_t)n, (uint32_t)(sms * tu.decCtasPerSm));
     DecArgs da{dBytes_, size, dCodes_, dBlocks_, (uint32_t)n, dHalf_, (uint32_t*)dPlanes_, (uint32_t)L_.width, dPerm_, dCtl_,
                grid, heavySms_ ? (uint32_t)tu.decHeavyPct : 0u};
-    orderKernel<<<1, 1024, 0, st>>>(da);
+    const uint32_t og = std::max(1u, std::min(divUp((uint32_t)n, 256u), (uint32_t)sms * 2u));
+    orderCountKernel<<<og, 256, 0, st>>>(da);
+    orderScatterKernel<<<og, 256, 0, st>>>(da);
     decodeKernel<<<grid, DEC_THREADS, 0, st>>>(da);
     GB_CHECK(cudaGetLastError());
     GB_CHECK(cudaEventRecord(ev_[1], st));

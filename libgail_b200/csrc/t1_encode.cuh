@@ -56,9 +56,9 @@ struct T1Launch {
     uint32_t* work;
 };
 
-// Words of a persistent launch's work area: control words and the order's buckets, then
-// one list entry per block.
-constexpr uint32_t kT1WorkHead = 16 + 128;
+// Words of a launch's work area: control words, the order's buckets and their cursors, then
+// (a persistent launch's) one list entry per block.
+constexpr uint32_t kT1WorkHead = 16 + 2 * 128;
 inline size_t t1WorkWords(uint32_t n) { return kT1WorkHead + (size_t)n; }
 
 // Enqueues the whole Tier-1 stage on st: context modelling, ordering, MQ coding and
