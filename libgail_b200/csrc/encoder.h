@@ -115,6 +115,7 @@ private:
     int32_t* hDist_ = nullptr;
     uint8_t* hData_ = nullptr;
     uint64_t hDataCap_ = 0;
+    uint64_t guessData_ = 0, guessPasses_ = 0;  // what encode() copies back before it knows the sizes
     float* hSlope_ = nullptr;
     // debug taps
     std::vector<uint16_t> xyz_;

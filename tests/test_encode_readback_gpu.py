@@ -1,0 +1,62 @@
+"""encoder_encode copies a frame's tables back before it knows their sizes, by those of the frame
+before: a frame that needs more than that (or less) comes out as from an encoder of its own. And
+t1_encode_blocks keeps its device memory between calls: a small call after a large one, and calls
+from several threads at once, give what each gives alone."""
+import threading
+
+import numpy as np
+import pytest
+
+import libgail_b200 as gb
+from libgail_b200 import plugin as P
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(1998, 1080), (64, 64)])
+def test_sizes_of_the_frame_before(w, h):
+    lay, fmt, col = P.LayoutHolder(w, h, 0), P.rgb48_format(w, h), P.color_passthrough()
+    rng = np.random.default_rng(3)
+    black, noise = np.zeros((h, w, 3), np.uint16), rng.integers(0, 65536, (h, w, 3)).astype(np.uint16)
+    soft = (30000 + 300 * rng.standard_normal((h, w, 3))).astype(np.uint16)
+    dev = P.Plugin().device(0)
+
+    def alone(f):
+        e = dev.encoder(lay, fmt, col)
+        t = e.encode(f)[0]
+        e.close()
+        return t
+
+    want = {k: alone(f) for k, f in (("black", black), ("noise", noise), ("soft", soft))}
+    enc = dev.encoder(lay, fmt, col)
+    for k in ("black", "noise", "soft", "noise", "black", "soft"):
+        got = enc.encode({"black": black, "noise": noise, "soft": soft}[k])[0]
+        for name in ("info", "pass_len", "pass_dist", "data"):
+            assert np.array_equal(getattr(got, name), getattr(want[k], name)), (k, name)
+    enc.close()
+    dev.close()
+
+
+@pytest.mark.gpu
+def test_blocks_memory_is_kept_safely():
+    rng = np.random.default_rng(5)
+    sets = []
+    for n in (300, 3, 40, 1):
+        c = np.minimum(16383, rng.exponential(900.0, (n, 1024))).astype(np.uint32)
+        sets.append((c, np.tile(np.array([32, 32, 1, 64], np.int32), (n, 1))))
+    want = [gb.t1_encode_blocks(*s, data_stride=4096) for s in sets]
+    got = [None] * 8
+
+    def call(i):
+        for _ in range(3):
+            got[i] = gb.t1_encode_blocks(*sets[i % len(sets)], data_stride=4096)
+
+    threads = [threading.Thread(target=call, args=(i,)) for i in range(len(got))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i, g in enumerate(got):
+        x = want[i % len(sets)]
+        coded = np.arange(64) < x[0][:, 1:2]
+        assert np.array_equal(g[0], x[0]) and g[3] == x[3]
+        assert np.array_equal(np.where(coded, g[1], 0), np.where(coded, x[1], 0))
