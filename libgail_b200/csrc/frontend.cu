@@ -199,8 +199,9 @@ __device__ __forceinline__ void dciCodes(const float* __restrict__ thr, const fl
         sure = sure && t[c][0] <= n[c] && t[c][3] > n[c];
         code[c] = b[c] - 1 + (t[c][1] <= n[c] ? 1 : 0) + (t[c][2] <= n[c] ? 1 : 0);
     }
-    if (!sure)
-#pragma unroll 1
+    if (!sure)  // rare, and unrolled: indexed by a loop, the arrays would live in local memory and
+                // every pixel would store them (4K PQ front end 0.372 ms against 0.308)
+#pragma unroll
         for (int c = 0; c < 3; ++c)
             if (!(t[c][0] <= n[c] && t[c][3] > n[c])) code[c] = dciCodeSearch(thr, n[c], b[c]);
 }
@@ -487,9 +488,10 @@ __host__ __device__ constexpr int feMinCtas() {
 // MODE 0: a later level from the previous LL planes; 1..3: level 1 with the colour route
 // of pixelCodes. SHAPE: the tile shape. Level 1 is bound by instruction issue (the colour
 // conversion of a tile and its halo), the later levels by latency. On a B200, the front end of a
-// 4K PQ frame 0.372 ms (0.401 with IEEE divisions, four chroma neighbours whatever the
+// 4K PQ frame 0.308 ms (0.401 with IEEE divisions, four chroma neighbours whatever the
 // subsampling, a pixel's thresholds one code after another, and 128 threads on a later level's
-// tile), of a 2K one 0.132 (0.167), of a 64 x 64 one 0.069 (0.104).
+// tile), of a 2K one 0.117 (0.167), of a 64 x 64 one 0.061 (0.104). Two or three pixels of
+// level 1 at once in a thread: 0.311, 0.331.
 template <int MODE, int SHAPE>
 __global__ void __launch_bounds__(feThreads<MODE, SHAPE>(), feMinCtas<MODE, SHAPE>())
     levelKernel(ColorArgs c, LevelArgs a) {
