@@ -103,10 +103,12 @@ GB_API int gb_color_route(const GailCudaColor* color, float* params48, int32_t* 
  * made after the call (plain encoders and decoders, engine batches). No counterpart in the
  * reference, whose launch shapes are fixed; libgail_b200/autotune.py measures candidates
  * on the GPU and keeps the fastest. gb_set_tuning(profile, NULL) restores the defaults.
- *   soloDecisions  MQ coding: blocks with at least this many decisions are coded alone in
- *                  a warp first (rounded down to a power of two; default 16384)
+ *   soloDecisions  MQ coding in launches of more than 128 blocks per scheduler (75,776 on
+ *                  148 SMs): blocks with at least this many decisions are coded alone in a
+ *                  warp first (rounded down to a power of two; default 16384). Smaller
+ *                  launches run a warp per scheduler and code their longest blocks alone.
  *   cmCtasPerSm, mqCtasPerSm, decCtasPerSm  grid caps in CTAs per SM of context modelling,
- *                  MQ coding and Tier-1 decoding (defaults 16, 16, 32; 1..64)
+ *                  MQ coding (such launches) and Tier-1 decoding (defaults 16, 16, 32; 1..64)
  *   t1Persistent   1: Tier-1 encoding as one persistent launch whose warps take context
  *                  modelling, the order, MQ coding and truncation lengths from device
  *                  queues in turn; 0 (default): four launches. Same results either way. */

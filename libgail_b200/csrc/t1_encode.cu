@@ -1142,19 +1142,28 @@ void t1Encode(const T1Launch& launch, cudaStream_t st, cudaEvent_t* marks) {
     const uint32_t cmBlocks = min(divUp(L.n, CM_WARPS), (uint32_t)sms * L.cmCtasPerSm);
     t1CmKernel<<<cmBlocks, CM_THREADS, 0, st>>>(L);
     if (marks) GB_CHECK(cudaEventRecord(marks[0], st));
-    // A wide (batched) launch gives each lane two blocks on average, so that lanes whose
-    // blocks end early take more from the queue.
-    const bool wide = divUp(L.n, MQ_THREADS) > (uint32_t)sms * 4u;
-    uint32_t mqBlocks = min(divUp(L.n, MQ_THREADS * (wide ? 2u : 1u)), (uint32_t)sms * L.mqCtasPerSm);
-    uint32_t maxSolo = mqBlocks * (MQ_THREADS / 32) / 2;
-    // A launch that does not fill one warp per scheduler is bound by its longest blocks: it
-    // gets that many warps, and as many of the longest blocks as leave a lane for every other
-    // block are coded alone (105 cycles a decision against 150 beside 31 others; a second warp
-    // on the scheduler costs a third more).
     const uint32_t warps = (uint32_t)sms * 4u;
-    if (L.n <= warps * 32u) {
-        mqBlocks = max(mqBlocks, min(divUp(L.n, MQ_THREADS / 32), warps / (MQ_THREADS / 32)));
-        maxSolo = (warps * 32u - L.n) / 31u;
+    const bool wide = divUp(L.n, MQ_THREADS) > warps;
+    uint32_t mqBlocks, maxSolo;
+    if (wide) {
+        // A wide (batched) launch gives each lane two blocks on average, so that lanes whose
+        // blocks end early take more from the queue; blocks of soloDecisions or more are coded
+        // alone, up to half the warps.
+        mqBlocks = min(divUp(L.n, MQ_THREADS * 2u), (uint32_t)sms * L.mqCtasPerSm);
+        maxSolo = mqBlocks * (MQ_THREADS / 32) / 2;
+    } else {
+        // A launch of a frame or a few is bound by its longest blocks' chains (105 cycles a
+        // decision alone in a warp, 150 beside 31 others, a third more with a second warp on the
+        // scheduler): one warp per scheduler while that leaves a lane at most one and a half
+        // blocks, else two, and the longest blocks alone first, as many as leave a lane for every
+        // other block or one for every twelve schedulers. 4K frame (25,986 blocks): 946 us; 1,105
+        // with a lane for each block and so a second warp on a third of the schedulers, 1,170 with
+        // no block alone, within 1 % of 946 from 16 to 96 of them alone. Two warps per scheduler
+        // and one, us: 26,000 blocks of 2K frames 1,006 and 1,019, 52,000 1,196 and 1,562, 71,000
+        // 1,501 and 2,067 (with a lane for each block 1,100, 1,658 and 1,838).
+        const uint32_t lanes = warps * 32u;
+        mqBlocks = min(divUp(L.n, MQ_THREADS / 32), (uint32_t)sms * (L.n > lanes + lanes / 2 ? 2u : 1u));
+        maxSolo = max(warps / 12u, L.n < lanes ? (lanes - L.n) / 31u : 0u);
         L.soloDecisions = 1;
     }
     if (L.work) {  // over the whole GPU: a batch of frames has 100,000 blocks and more

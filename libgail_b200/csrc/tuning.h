@@ -8,8 +8,9 @@ namespace gb {
 
 struct Tuning {
     uint32_t soloDecisions = 16384;  // MQ: blocks with at least this many decisions coded alone in a warp
+                                     // (launches of more than 128 blocks per scheduler)
     int cmCtasPerSm = 16;            // context modelling grid cap
-    int mqCtasPerSm = 16;            // MQ grid cap
+    int mqCtasPerSm = 16;            // MQ grid cap of the same launches
     int decCtasPerSm = 32;           // Tier-1 decode grid cap
     int t1Persistent = 0;            // Tier-1 encode as one persistent launch (1) or four (0)
     int decHeavyPct = 150;           // Tier-1 decode: blocks above this % of the mean codeword bytes per

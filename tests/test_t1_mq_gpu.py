@@ -10,7 +10,7 @@ from oracle.oracle import Oracle
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,size,planes", [(1, 32, 12), (33, 32, 14), (700, 32, 9), (19000, 8, 12), (76000, 8, 9)])
+@pytest.mark.parametrize("n,size,planes", [(1, 32, 12), (33, 32, 14), (700, 32, 9), (18900, 8, 12), (19000, 8, 12), (76000, 8, 9)])
 def test_mq_matches_oracle(n, size, planes):
     rng = np.random.default_rng(n)
     top = 1 << (planes + 6)
