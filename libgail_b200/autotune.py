@@ -188,6 +188,8 @@ def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
             log(f"[{name}] front-end tile shapes (front-end ms per frame)")
             tiles = {"dwtTile1": [1, 2], "dwtTileN": [1, 2]}
             cfg, _, seen0 = coordinate_search(cfg, tiles, _best_of(front_ms, runs), log=log)
+            # one-frame launches use it in the persistent form only: their separate MQ launch
+            # has a rule of its own
             log(f"[{name}] MQ solo threshold (Tier-1 ms per frame)")
             solo = {"soloDecisions": [4096, 8192, 32768, 1 << 30]}
             cfg, _, seen1 = coordinate_search(cfg, solo, _best_of(tier1_ms, runs), log=log)

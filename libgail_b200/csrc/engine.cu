@@ -1064,10 +1064,9 @@ bool EncodeEngine::launchBatch(Batch& b) {
     bool any4k = false;  // a batch with a 4K frame is launched with the 4K tuning
     for (Request* r : sel) any4k = any4k || classes_[r->cls]->L.profile == 1;
     const Tuning tu = tuningFor(any4k ? 1 : 0);
-    // the solo threshold is tuned on one-frame launches, where the longest blocks' chains set
-    // the time; a batch of frames has enough other blocks to hide them behind, and taking
-    // warps for solo blocks below 16,384 decisions cost it throughput (4K served codestreams:
-    // 560 per second at 16,384, 530 at 8,192, on B200)
+    // A batch of frames has enough other blocks to hide the longest ones' chains behind: taking
+    // warps for solo blocks below 16,384 decisions gave it nothing (24 4K frames on a B200
+    // 30.2-31.0 ms whatever the number of solo blocks up to 200) or cost it throughput
     L.soloDecisions = std::max<uint32_t>(tu.soloDecisions, kBatchSoloFloor);
     L.cmCtasPerSm = (uint16_t)tu.cmCtasPerSm;
     L.mqCtasPerSm = (uint16_t)tu.mqCtasPerSm;
