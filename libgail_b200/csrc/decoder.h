@@ -29,9 +29,10 @@ void decoderInit();
 
 class DecoderSlot {
 public:
-    // heavySms: decode the heaviest code-blocks on SMs of their own (the tuning's decHeavyPct),
-    // for a decode that has the GPU to itself; slots of which several decode at once (the
-    // served engine's) leave it off, as their launches would all reserve the same SMs.
+    // heavySms: decode the heaviest code-blocks on SMs of their own (the tuning's decHeavyPct)
+    // whenever no other decode of this process is in flight on the device; slots of which several
+    // decode at once (the served engine's) leave it off, as their launches would all reserve the
+    // same SMs.
     DecoderSlot(int device, const Layout& L, const GailCudaDecodeSettings& s, bool heavySms = true);
     ~DecoderSlot();
     DecoderSlot(const DecoderSlot&) = delete;
@@ -55,11 +56,13 @@ public:
 
 private:
     void release();
+    void ended();  // this slot's decode, if one is counted, is no longer in flight
     int dev_;
     Layout L_;
     GailCudaDecodeSettings s_;
     int outW_ = 0, outH_ = 0;
     bool heavySms_ = true;
+    bool counted_ = false;
     cudaStream_t st_ = nullptr;
     cudaEvent_t ev_[4] = {};
     static constexpr int kBands = 8;
