@@ -14,6 +14,7 @@
 #include "gail_b200.h"
 #include "common.cuh"
 #include "compact.cuh"
+#include "pack_runs.h"
 #include "t1_encode.cuh"
 
 using namespace gb;
@@ -42,6 +43,10 @@ Kept& keptOnThisDevice() {
     if (dev < 0 || dev >= kMaxDevices) throw std::runtime_error("device index out of range");
     return kept[dev];
 }
+
+// Codewords come back packed, in runs of at most this many bytes: packed offsets are 32 bits, and a
+// call's codewords may be more.
+constexpr uint64_t kRunBytes = 64u << 20;
 
 // One piece of device memory in parts, each 256-byte aligned: first the parts' offsets, then the
 // memory.
@@ -138,37 +143,41 @@ GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uin
         T1Launch L{d.at<T1Job>(oJobs), n, d.at<uint32_t>(oInfo), d.at<uint32_t>(oEnd), d.at<uint32_t>(oLen),
                    d.at<int32_t>(oDist), d.at<uint4>(oSnaps), d.at<uint32_t>(oPerm), ctl, d.at<float>(oSlope)};
         t1Encode(L, 0);
-        // the packed codewords where the decisions were, the packed pass lengths (not read back:
-        // the caller's tables have a row per block) where the MQ states were
-        CompactArgs ca{};
-        ca.n = n;
-        ca.info = d.at<uint32_t>(oInfo);
-        ca.passLen = d.at<uint32_t>(oLen);
-        ca.passDist = d.at<int32_t>(oDist);
-        ca.jobs = d.at<T1Job>(oJobs);
-        ca.outInfo = d.at<uint32_t>(oOutInfo);
-        ca.outPassLen = d.at<uint32_t>(oSnaps);
-        ca.outData = d.at<uint8_t>(oSym);
-        ca.tot = ctl + 8;
-        ca.dataCap = region;
-        ca.scratch = d.at<uint32_t>(oPerm);
-        ca.offsets = d.at<uint2>(oOffsets);
-        compactTier1(ca, 0);
+        // a run's packed codewords where the decisions were
+        auto pack = [&](uint32_t first, uint32_t count) {
+            CompactArgs ca{};
+            ca.n = count;
+            ca.info = d.at<uint32_t>(oInfo) + 4 * (size_t)first;
+            ca.jobs = d.at<T1Job>(oJobs) + first;
+            ca.outInfo = d.at<uint32_t>(oOutInfo);
+            ca.outData = d.at<uint8_t>(oSym);
+            ca.tot = ctl + 8;
+            ca.dataCap = region;
+            ca.scratch = d.at<uint32_t>(oPerm);
+            ca.offsets = d.at<uint2>(oOffsets);
+            compactTier1(ca, 0);
+        };
+        const bool whole = region <= kRunBytes;  // one run whatever the codewords' lengths
+        if (whole) pack(0, n);
         uint32_t words[16];
         GB_CHECK(cudaMemcpy(words, ctl, 64, cudaMemcpyDeviceToHost));  // waits for the kernels
         if (words[1]) throw std::runtime_error("Tier-1 encoder status " + std::to_string(words[1]));
         GB_CHECK(cudaMemcpy(info4, d.at<void>(oInfo), 16 * (size_t)n, cudaMemcpyDeviceToHost));
         GB_CHECK(cudaMemcpy(passLen, d.at<void>(oLen), tables, cudaMemcpyDeviceToHost));
         GB_CHECK(cudaMemcpy(passDist, d.at<void>(oDist), tables, cudaMemcpyDeviceToHost));
-        const uint32_t total = words[8];
-        const std::unique_ptr<uint8_t[]> cw(new uint8_t[total + 1]);
-        if (total) GB_CHECK(cudaMemcpy(cw.get(), d.at<void>(oSym), total, cudaMemcpyDeviceToHost));
-        size_t at = 0;  // block i's codeword, each on a 4-byte boundary
-        for (uint32_t i = 0; i < n; ++i) {
-            const uint32_t len = info4[4 * i + 3];
-            if (len > dataStride) throw std::logic_error("dataStride too small for a codeword");
-            std::memcpy(data + (size_t)i * dataStride, cw.get() + at, len);
-            at += (len + 3u) & ~3u;
+        for (uint32_t first = 0, end; first < n; first = end) {
+            uint64_t total = 0;
+            end = packedRun(info4, first, n, kRunBytes, total);
+            if (!whole) pack(first, end - first);
+            const std::unique_ptr<uint8_t[]> cw(new uint8_t[total + 1]);
+            if (total) GB_CHECK(cudaMemcpy(cw.get(), d.at<void>(oSym), total, cudaMemcpyDeviceToHost));
+            size_t at = 0;  // block i's codeword, each on a 4-byte boundary
+            for (uint32_t i = first; i < end; ++i) {
+                const uint32_t len = info4[4 * (size_t)i + 3];
+                if (len > dataStride) throw std::logic_error("dataStride too small for a codeword");
+                std::memcpy(data + (size_t)i * dataStride, cw.get() + at, len);
+                at += (len + 3u) & ~3u;
+            }
         }
     });
 }

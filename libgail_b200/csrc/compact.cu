@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) copyKernel(CompactArgs a) {
         const uint32_t np = in.y, len = in.w;
         const size_t src = (size_t)blk * kMaxPasses;
         for (uint32_t q = lane; q < np; q += 32) {
-            a.outPassLen[o.y + q] = a.passLen[src + q];
+            if (a.outPassLen) a.outPassLen[o.y + q] = a.passLen[src + q];
             if (a.outPassDist) a.outPassDist[o.y + q] = a.passDist[src + q];
         }
         if (a.outHullPasses)

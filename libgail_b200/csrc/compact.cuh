@@ -15,7 +15,7 @@ struct CompactArgs {
     const int32_t* passDist;   // 64 per block
     const T1Job* jobs;         // each block's codeword region
     uint32_t* outInfo;         // 5 words per block: CblkInfo
-    uint32_t* outPassLen;
+    uint32_t* outPassLen;      // may be null: no pass lengths
     int32_t* outPassDist;      // may be null: no distortions
     uint8_t* outData;
     uint32_t* tot;             // [0] data bytes, [1] passes, [2] set when outData was too small
