@@ -47,13 +47,15 @@ GB_API const char* gb_last_error(void);
  *   slope      early-termination threshold (0: code every pass)
  *   distScale  per-block distortion scale of that rule (NULL: 1)
  *   info4      out: n x {nbps, passes, MQ decisions, codeword bytes}
- *   passLen    out: n x 64 truncation lengths; passDist: n x 64 distortion reductions
+ *   passLen    out: n x 64 truncation lengths; passDist: n x 64 distortion reductions (0 past a
+ *              block's passes)
  *   data       out: codeword of block i at data + i * dataStride */
 GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uint32_t n, float slope,
                                const float* distScale, uint32_t* info4, uint32_t* passLen, int32_t* passDist,
                                uint8_t* data, uint32_t dataStride);
 
-/* gb_t1_encode_blocks without any allocation. No counterpart in the reference: it is for
+/* gb_t1_encode_blocks without any allocation (its tables past a block's passes are left
+ * undefined). No counterpart in the reference: it is for
  * callers that must not allocate device memory themselves, such as a real-time frame
  * thread (cudaMalloc may wait for the whole device and stall it) or a process whose
  * device memory is budgeted up front. Same arguments and results as gb_t1_encode_blocks,

@@ -139,6 +139,9 @@ GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uin
         GB_CHECK(cudaMemcpy(d.at<void>(oJobs), jobs.data(), n * sizeof(T1Job), cudaMemcpyHostToDevice));
         GB_CHECK(cudaMemcpy(d.at<void>(oSlope), &slope, 4, cudaMemcpyHostToDevice));
         GB_CHECK(cudaMemset(d.at<void>(oCtl), 0, 64));
+        // the kernels write a block's passes alone; the rest of its rows is 0, not what a call before left
+        GB_CHECK(cudaMemset(d.at<void>(oLen), 0, tables));
+        GB_CHECK(cudaMemset(d.at<void>(oDist), 0, tables));
         uint32_t* const ctl = d.at<uint32_t>(oCtl);
         T1Launch L{d.at<T1Job>(oJobs), n, d.at<uint32_t>(oInfo), d.at<uint32_t>(oEnd), d.at<uint32_t>(oLen),
                    d.at<int32_t>(oDist), d.at<uint4>(oSnaps), d.at<uint32_t>(oPerm), ctl, d.at<float>(oSlope)};
