@@ -54,6 +54,12 @@ GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uin
                                const float* distScale, uint32_t* info4, uint32_t* passLen, int32_t* passDist,
                                uint8_t* data, uint32_t dataStride);
 
+/* Gives back the device memory that gb_t1_encode_blocks keeps on the current device between calls
+ * (up to 64 MB: what the last call used, idle in between). It is given back too when another
+ * allocation of this library's finds the device out of memory; cudaDeviceReset is not supported
+ * once this library has been used on the device. No counterpart in the reference. */
+GB_API int gb_t1_release_memory(void);
+
 /* gb_t1_encode_blocks without any allocation (its tables past a block's passes are left
  * undefined). No counterpart in the reference: it is for
  * callers that must not allocate device memory themselves, such as a real-time frame

@@ -23,8 +23,9 @@ namespace {
 
 // The memory of the call before, one block per device, kept for the next call up to kKeepBytes:
 // taken by one call at a time (another allocates its own), replaced by a larger one, given back
-// when the library is unloaded. A call waits for its kernels before it returns, so the memory is
-// idle in between.
+// when an allocation of the library's fails for want of memory, by gb_t1_release_memory and when
+// the library is unloaded. A call waits for its kernels before it returns, so the memory is idle
+// in between.
 constexpr size_t kKeepBytes = 64u << 20;
 constexpr int kMaxDevices = 64;
 struct Kept {
@@ -42,6 +43,21 @@ Kept& keptOnThisDevice() {
     GB_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) throw std::runtime_error("device index out of range");
     return kept[dev];
+}
+
+// Gives back what is kept on this device, if no call is using it.
+bool giveBack() {
+    Kept& k = keptOnThisDevice();
+    uint8_t* drop = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(k.m);
+        if (k.taken || !k.p) return false;
+        drop = k.p;
+        k.p = nullptr;
+        k.size = 0;
+    }
+    GB_CHECK(cudaFree(drop));
+    return true;
 }
 
 // Codewords come back packed, in runs of at most this many bytes: packed offsets are 32 bits, and a
@@ -66,7 +82,7 @@ public:
                 return;
             }
         }
-        GB_CHECK(cudaMalloc((void**)&base_, size_));
+        GB_CHECK(deviceAlloc((void**)&base_, size_));
     }
     template <class T>
     T* at(size_t offset) const {
@@ -100,7 +116,20 @@ private:
 
 }  // namespace
 
+cudaError_t gb::deviceAlloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && giveBack()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 extern "C" {
+
+GB_API int gb_t1_release_memory(void) {
+    return gbGuard([] { giveBack(); });
+}
 
 GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uint32_t n, float slope, const float* distScale,
                         uint32_t* info4, uint32_t* passLen, int32_t* passDist, uint8_t* data, uint32_t dataStride) {

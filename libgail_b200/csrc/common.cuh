@@ -42,6 +42,10 @@ inline void check(cudaError_t e, const char* what) {
 
 #define GB_CHECK(x) ::gb::check((x), #x)
 
+// cudaMalloc for the library's own memory: when the device is out of it, what t1_encode_blocks keeps
+// between calls (capi_blocks.cu) is given back first.
+cudaError_t deviceAlloc(void** p, size_t bytes);
+
 __host__ __device__ inline uint32_t divUp(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 }  // namespace gb

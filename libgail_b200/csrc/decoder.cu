@@ -767,7 +767,7 @@ DecoderSlot::DecoderSlot(int device, const Layout& L, const GailCudaDecodeSettin
         const uint64_t n = (uint64_t)L.numCblks();
         auto alloc = [&](auto*& p, uint64_t bytes) {
             void* q = nullptr;
-            check(cudaMalloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a decoder slot");
+            check(deviceAlloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a decoder slot");
             allocs_.push_back(q);
             p = static_cast<std::remove_reference_t<decltype(p)>>(q);
         };
@@ -888,7 +888,7 @@ void DecoderSlot::enqueue(const Layout& frame, const uint8_t* data, size_t size,
         hBytes_ = nullptr;
         capBytes_ = size + size / 2;
         void* q = nullptr;
-        check(cudaMalloc(&q, capBytes_), "device memory for a decoder slot");
+        check(deviceAlloc(&q, capBytes_), "device memory for a decoder slot");
         dBytes_ = (uint8_t*)q;
         allocs_.push_back(q);
         check(cudaHostAlloc((void**)&hBytes_, capBytes_, cudaHostAllocDefault), "pinned host memory");

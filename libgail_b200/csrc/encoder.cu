@@ -152,7 +152,7 @@ EncoderSlot::EncoderSlot(int device, const Layout& L, const GailCudaEncodeSettin
         for (auto& e : ev_) GB_CHECK(cudaEventCreate(&e));
         auto alloc = [&](auto*& p, uint64_t bytes) {
             void* q = nullptr;
-            check(cudaMalloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for an encoder slot");
+            check(deviceAlloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for an encoder slot");
             dev_allocs_.push_back(q);
             p = static_cast<std::remove_reference_t<decltype(p)>>(q);
         };
@@ -335,8 +335,8 @@ void EncoderSlot::encode(const void* frame, GailCudaTier1* out, GbFrameTimings* 
     if (!frame) throw std::logic_error("no frame");
     const bool full = dbg && dbg->full;
     const uint64_t npix = z_.npix, n = z_.n;
-    if (dbg && !dXyz_) check(cudaMalloc(&dXyz_, npix * 6), "device memory for the debug taps");
-    if (full && !dTap_) check(cudaMalloc(&dTap_, npix * 12), "device memory for the debug taps");
+    if (dbg && !dXyz_) check(deviceAlloc((void**)&dXyz_, npix * 6), "device memory for the debug taps");
+    if (full && !dTap_) check(deviceAlloc((void**)&dTap_, npix * 12), "device memory for the debug taps");
     if (frame != hIn_) std::memcpy(hIn_, frame, z_.inBytes);
     *hSlope_ = slope_;
     const cudaStream_t st = st_;

@@ -170,7 +170,7 @@ EncodeEngine::EncodeEngine(int device, uint64_t hbmBudget, int maxBatch) : dev_(
     budget_ = hbmBudget;
     for (auto& f : front_) GB_CHECK(cudaStreamCreateWithFlags(&f, cudaStreamNonBlocking));
     GB_CHECK(cudaStreamCreateWithFlags(&copy_, cudaStreamNonBlocking));
-    check(cudaMalloc(&dSlope_, kMaxSlots * 4), "device memory for the engine");
+    check(deviceAlloc((void**)&dSlope_, kMaxSlots * 4), "device memory for the engine");
     check(cudaHostAlloc((void**)&hSlope_, kMaxSlots * 4, cudaHostAllocDefault), "pinned host memory");
     check(cudaHostAlloc((void**)&hZero_, 16, cudaHostAllocDefault), "pinned host memory");
     *hZero_ = 0.f;
@@ -242,7 +242,7 @@ int EncodeEngine::addClass(const GailCudaLayout& layout, const GailCudaEncodeSet
     c->color = buildColorTables(s.color);
     auto alloc = [&](auto*& p, uint64_t bytes) {
         void* q = nullptr;
-        check(cudaMalloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for the engine");
+        check(deviceAlloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for the engine");
         c->dev.push_back(q);
         p = static_cast<std::remove_reference_t<decltype(p)>>(q);
     };
@@ -325,7 +325,7 @@ void EncodeEngine::growBatch(Batch& b, uint64_t blocks, uint64_t poolBytes) {
         const uint64_t cap = blocks;
         auto alloc = [&](auto*& p, uint64_t bytes) {
             void* q = nullptr;
-            check(cudaMalloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a Tier-1 batch");
+            check(deviceAlloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a Tier-1 batch");
             b.dev.push_back(q);
             p = static_cast<std::remove_reference_t<decltype(p)>>(q);
         };
@@ -349,10 +349,10 @@ void EncodeEngine::growBatch(Batch& b, uint64_t blocks, uint64_t poolBytes) {
         b.poolCap = 0;
         b.symPool = b.cwPool = nullptr;
         void* q = nullptr;
-        check(cudaMalloc(&q, poolBytes), "device memory for a Tier-1 batch's decision pool");
+        check(deviceAlloc(&q, poolBytes), "device memory for a Tier-1 batch's decision pool");
         b.pools.push_back(q);
         b.symPool = static_cast<uint8_t*>(q);
-        check(cudaMalloc(&q, poolBytes), "device memory for a Tier-1 batch's codeword pool");
+        check(deviceAlloc(&q, poolBytes), "device memory for a Tier-1 batch's codeword pool");
         b.pools.push_back(q);
         b.cwPool = static_cast<uint8_t*>(q);
         b.poolCap = poolBytes;
@@ -445,7 +445,7 @@ EncodeEngine::Slot* EncodeEngine::newSlot(int cls) {
     s->n = (uint32_t)c.z.n;
     auto alloc = [&](auto*& p, uint64_t bytes) {
         void* q = nullptr;
-        check(cudaMalloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a frame slot");
+        check(deviceAlloc(&q, std::max<uint64_t>(bytes, 16)), "device memory for a frame slot");
         s->dev.push_back(q);
         p = static_cast<std::remove_reference_t<decltype(p)>>(q);
     };

@@ -484,7 +484,7 @@ struct DevBuf {  // a growable device buffer
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        check(cudaMalloc((void**)&p, std::max<size_t>(n, 16) * sizeof(T)), "device memory for rate control");
+        check(deviceAlloc((void**)&p, std::max<size_t>(n, 16) * sizeof(T)), "device memory for rate control");
         cap = n;
     }
     ~DevBuf() {

@@ -1,11 +1,13 @@
 """encoder_encode copies a frame's tables back before it knows their sizes, by those of the frame
 before: a frame that needs more than that (or less) comes out as from an encoder of its own. And
 t1_encode_blocks keeps its device memory between calls: a small call after a large one, and calls
-from several threads at once, give what each gives alone."""
+from several threads at once, give what each gives alone, and it is given back when it is asked
+for or needed elsewhere."""
 import threading
 
 import numpy as np
 import pytest
+import torch
 
 import libgail_b200 as gb
 from libgail_b200 import plugin as P
@@ -62,3 +64,28 @@ def test_blocks_memory_is_kept_safely():
         for k in (1, 2):
             assert np.array_equal(g[k], x[k])
             assert not g[k][past].any()
+
+
+@pytest.mark.gpu
+def test_kept_memory_is_given_back():
+    def call(n):
+        c = np.full((n, 1024), 64, np.uint32)
+        return gb.t1_encode_blocks(c, np.tile(np.array([32, 32, 0, 64], np.int32), (n, 1)), data_stride=4096)
+
+    mb = 1 << 20
+    gb.check(gb.lib().gb_t1_release_memory())
+    call(1)  # whatever a first call loads
+    gb.check(gb.lib().gb_t1_release_memory())
+    free = torch.cuda.mem_get_info()[0]
+    want = call(500)  # 59 MB, kept
+    assert free - torch.cuda.mem_get_info()[0] >= 48 * mb
+    gb.check(gb.lib().gb_t1_release_memory())
+    assert free - torch.cuda.mem_get_info()[0] < 4 * mb
+    call(500)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - 90 * mb, dtype=torch.uint8, device="cuda")
+    try:
+        got = call(1000)  # 119 MB: only with the 59
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert got[3] == want[3] * 2
