@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decodeKernel(DecArgs a)
 #pragma unroll
             for (int r = 0; r < 32; ++r)
                 if (r < h) {
-                    const float mag = (float)(v[r] & 0x7FFFFFFFu) * half;
+                    // 0 stays 0 whatever the step (an infinite one included)
+                    const float mag = v[r] ? (float)(v[r] & 0x7FFFFFFFu) * half : 0.f;
                     out[(size_t)r * a.W] = (v[r] & 0x80000000u) ? -mag : mag;
                 }
         }

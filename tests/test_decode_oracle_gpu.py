@@ -98,3 +98,21 @@ def test_planes_match_oracle(dev, w, h, fourk, how):
     want = _planes(lay, b, data.tobytes())
     assert np.array_equal(wl.reshape(3, h, w).view(np.uint32) & 0x7FFFFFFF, want.view(np.uint32) & 0x7FFFFFFF)
     assert np.array_equal(wl.reshape(3, h, w), want)
+
+
+@pytest.mark.gpu
+def test_insignificant_samples_are_zero_whatever_the_step(dev):
+    w, h = 130, 65
+    cs = _codestream(dev, w, h, 0, 20.0)
+    lay, b = CS.parse(cs)
+    b = b.view(P.CBLK_CODE_DTYPE).copy()
+    sound = _planes(lay, b, cs)
+    for band in lay.bands:
+        band.delta = float("inf")
+    dec = dev.decoder(lay)
+    _, _, wl = dec.decode(cs, b, frame_layout=lay, wavelet=True)
+    dec.close()
+    zero = sound == 0
+    assert 0.01 < zero.mean() < 0.99
+    assert not wl.reshape(3, h, w)[zero].any()  # NaN counts as any
+    assert not np.isfinite(wl.reshape(3, h, w)[~zero]).any()
