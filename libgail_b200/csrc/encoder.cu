@@ -118,9 +118,9 @@ void launchFrontEnd(const Layout& L, const ColorArgs& c, float* ll0, float* ll1,
     }
 }
 
-// A packed frame's tables up to this size are copied back whole: a bus transfer of it takes less
-// than finding out the sizes first.
-constexpr uint64_t kWholeBytes = 512 << 10;
+// What encode() copies back before it knows a frame's sizes: 2 MB and 512 KB are 50 us of the bus, a
+// little more than the host takes to read the sizes and ask for the rest.
+constexpr uint64_t kAheadData = 2 << 20, kAheadPasses = 64 << 10;
 
 SlotSizes slotSizes(const Layout& L, const GbFrameFormat& in) {
     SlotSizes z;
@@ -196,8 +196,6 @@ EncoderSlot::EncoderSlot(int device, const Layout& L, const GailCudaEncodeSettin
         pinned(hSlope_, 16);
         hDataCap_ = std::min<uint64_t>(z_.arena, std::max<uint64_t>(64ull << 20, n * 2048));
         pinned(hData_, hDataCap_);
-        guessData_ = std::min<uint64_t>(z_.outCap, std::max<uint64_t>(kWholeBytes, z_.npix * 9 / 4));
-        guessPasses_ = n * std::min<uint64_t>(kMaxPasses, std::max<uint64_t>(20, kWholeBytes / (8 * n)));
         uploadStatic();
     } catch (...) {
         release();
@@ -346,43 +344,40 @@ void EncoderSlot::encode(const void* frame, GailCudaTier1* out, GbFrameTimings* 
     GB_CHECK(cudaMemsetAsync(dCtl_ + 1, 0, 4, st));
     GB_CHECK(cudaEventRecord(ev_[1], st));
     enqueueStages(dIn_, dbg != nullptr, full);
-    // The packed frame's sizes are known on the device alone: the copies start at once, with the last
-    // frame's sizes and a sixteenth more (or small tables whole), and what that leaves out follows.
-    // A round trip to the host for the sizes first took 0.1-0.3 ms of each frame on a B200 (a 64 x 64
-    // frame 1.27 ms, now 1.06; a 4K one 4.34, now 4.10).
-    const uint64_t gotData = std::min(guessData_, hDataCap_), gotPasses = guessPasses_;
+    // The packed frame's sizes are known on the device alone. They are copied first, and while the
+    // host waits for them the bus carries on with what nearly every frame has, at most kAhead*; the
+    // rest follows by the sizes. A round trip for the sizes before anything else took 0.1-0.3 ms of
+    // each frame on a B200 (a 64 x 64 frame 1.27 ms, 1.06 so), and copying as much as the frame
+    // before had cost a flat 4K frame after a noisy one 0.9 ms of 2.5.
+    const uint64_t aheadData = std::min({kAheadData, z_.outCap, hDataCap_}), aheadPasses = std::min(kAheadPasses, n * kMaxPasses);
     GB_CHECK(cudaMemcpyAsync(hSmall_, dCtl_, 64, cudaMemcpyDeviceToHost, st));
+    GB_CHECK(cudaEventRecord(ev_[5], st));
     GB_CHECK(cudaMemcpyAsync(hInfo_, dOutInfo_, n * 20, cudaMemcpyDeviceToHost, st));
-    GB_CHECK(cudaMemcpyAsync(hLen_, dOutLen_, gotPasses * 4, cudaMemcpyDeviceToHost, st));
-    GB_CHECK(cudaMemcpyAsync(hDist_, dOutDist_, gotPasses * 4, cudaMemcpyDeviceToHost, st));
-    GB_CHECK(cudaMemcpyAsync(hData_, dOutData_, gotData, cudaMemcpyDeviceToHost, st));
-    GB_CHECK(cudaEventRecord(ev_[4], st));
-    GB_CHECK(cudaStreamSynchronize(st));
+    GB_CHECK(cudaMemcpyAsync(hLen_, dOutLen_, aheadPasses * 4, cudaMemcpyDeviceToHost, st));
+    GB_CHECK(cudaMemcpyAsync(hDist_, dOutDist_, aheadPasses * 4, cudaMemcpyDeviceToHost, st));
+    GB_CHECK(cudaMemcpyAsync(hData_, dOutData_, aheadData, cudaMemcpyDeviceToHost, st));
+    GB_CHECK(cudaEventSynchronize(ev_[5]));
     const uint32_t status = hSmall_[1], totData = hSmall_[8], totPasses = hSmall_[9];
     if (status) throw std::runtime_error("Tier-1 kernels reported status " + std::to_string(status));
-    uint64_t fromData = std::min<uint64_t>(gotData, totData);
+    uint64_t fromData = aheadData;
     if (totData > hDataCap_) {
+        GB_CHECK(cudaStreamSynchronize(st));  // the copy into it is done
         cudaFreeHost(hData_);
         hData_ = nullptr;
         hDataCap_ = (uint64_t)totData + totData / 2;
         check(cudaHostAlloc((void**)&hData_, hDataCap_, cudaHostAllocDefault), "pinned host memory");
         fromData = 0;
     }
-    if (totPasses > gotPasses || totData > fromData) {
-        if (totPasses > gotPasses) {
-            const uint64_t more = (totPasses - gotPasses) * 4;
-            GB_CHECK(cudaMemcpyAsync(hLen_ + gotPasses, dOutLen_ + gotPasses, more, cudaMemcpyDeviceToHost, st));
-            GB_CHECK(cudaMemcpyAsync(hDist_ + gotPasses, dOutDist_ + gotPasses, more, cudaMemcpyDeviceToHost, st));
-        }
-        if (totData > fromData)
-            GB_CHECK(cudaMemcpyAsync(hData_ + fromData, dOutData_ + fromData, totData - fromData, cudaMemcpyDeviceToHost, st));
-        GB_CHECK(cudaEventRecord(ev_[4], st));
-        GB_CHECK(cudaStreamSynchronize(st));
+    if (totPasses > aheadPasses) {
+        const uint64_t more = (totPasses - aheadPasses) * 4;
+        GB_CHECK(cudaMemcpyAsync(hLen_ + aheadPasses, dOutLen_ + aheadPasses, more, cudaMemcpyDeviceToHost, st));
+        GB_CHECK(cudaMemcpyAsync(hDist_ + aheadPasses, dOutDist_ + aheadPasses, more, cudaMemcpyDeviceToHost, st));
     }
+    if (totData > fromData)
+        GB_CHECK(cudaMemcpyAsync(hData_ + fromData, dOutData_ + fromData, totData - fromData, cudaMemcpyDeviceToHost, st));
+    GB_CHECK(cudaEventRecord(ev_[4], st));
+    GB_CHECK(cudaStreamSynchronize(st));
     GB_CHECK(cudaGetLastError());
-    guessData_ = std::min<uint64_t>(z_.outCap, std::max<uint64_t>(kWholeBytes, (uint64_t)totData + totData / 16));
-    guessPasses_ = std::min<uint64_t>(n * kMaxPasses,
-                                      std::max<uint64_t>(kWholeBytes / 8, (uint64_t)totPasses + totPasses / 16));
 
     *out = {reinterpret_cast<const GbCblkInfo*>(hInfo_), hLen_, hDist_, hData_, n, totPasses, totData};
     if (dbg) {

@@ -89,7 +89,7 @@ private:
     SlotSizes z_;
     float slope_ = 0.f;
     cudaStream_t st_ = nullptr;
-    cudaEvent_t ev_[5] = {};
+    cudaEvent_t ev_[6] = {};  // around a frame's stages; [5]: its packed sizes are in host memory
     bool timing_ = false;
     std::vector<cudaEvent_t> ring_;  // kTimingRing x 6 events
     int ringNext_ = 0, ringCount_ = 0;
@@ -115,7 +115,6 @@ private:
     int32_t* hDist_ = nullptr;
     uint8_t* hData_ = nullptr;
     uint64_t hDataCap_ = 0;
-    uint64_t guessData_ = 0, guessPasses_ = 0;  // what encode() copies back before it knows the sizes
     float* hSlope_ = nullptr;
     // debug taps
     std::vector<uint16_t> xyz_;

@@ -1,5 +1,6 @@
-"""encoder_encode copies a frame's tables back before it knows their sizes, by those of the frame
-before: a frame that needs more than that (or less) comes out as from an encoder of its own. And
+"""encoder_encode copies part of a frame's tables back before it knows their sizes: a frame that needs
+more than that (or less) comes out as from an encoder of its own, whatever the frame before it was,
+and takes the bus no longer. And
 t1_encode_blocks keeps its device memory between calls: a small call after a large one, and calls
 from several threads at once, give what each gives alone, and it is given back when it is asked
 for or needed elsewhere."""
@@ -36,6 +37,20 @@ def test_sizes_of_the_frame_before(w, h):
             assert np.array_equal(getattr(got, name), getattr(want[k], name)), (k, name)
     enc.close()
     dev.close()
+
+
+@pytest.mark.gpu
+def test_a_light_frame_after_a_heavy_one_copies_little():
+    w, h = 3996, 2160
+    enc = (dev := P.Plugin().device(0)).encoder(P.LayoutHolder(w, h, 1), P.rgb48_format(w, h), P.color_passthrough())
+    noise, flat = np.random.default_rng(3).integers(0, 65536, (h, w, 3)).astype(np.uint16), np.zeros((h, w, 3), np.uint16)
+    ms = {"noise": [], "flat": []}
+    for _ in range(3):
+        ms["noise"].append(enc.encode(noise)[1].download)  # 40 MB
+        ms["flat"].append(enc.encode(flat)[1].download)  # next to nothing
+    enc.close()
+    dev.close()
+    assert max(ms["flat"]) < 0.5 * min(ms["noise"]), ms
 
 
 @pytest.mark.gpu
