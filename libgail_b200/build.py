@@ -21,8 +21,11 @@ LIB = os.path.join(HERE, "libgail_cuda13.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden", "--fmad=false",
-          "-I", CSRC, "-I", INCLUDE]
+# Host functions start on cache lines, so that their speed does not depend on the size of what is
+# linked before them (32 served 2K frames with codestreams: 18.3-18.6 ms whatever the other objects,
+# 18.3-19.0 without).
+COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden,-falign-functions=64",
+          "--fmad=false", "-I", CSRC, "-I", INCLUDE]
 # exported: the plugin entry point and the gb_* C API (include/*.h), nothing else (no
 # template instantiations of the C++ standard library, nothing of the static CUDA runtime)
 EXPORTS = os.path.join(CSRC, "exports.map")
@@ -35,15 +38,16 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
-def _headers_mtime() -> float:
-    hs = glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + \
+def _shared_mtime() -> float:
+    """The newest of the headers and this file, which every object depends on."""
+    hs = [os.path.abspath(__file__)] + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + \
         glob.glob(os.path.join(INCLUDE, "*.h"))
-    return max((os.path.getmtime(h) for h in hs), default=0.0)
+    return max(os.path.getmtime(h) for h in hs)
 
 
 def _compile(src: str, verbose_ptxas: bool) -> str:
     obj = os.path.join(OUT, os.path.basename(src) + ".o")
-    if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(src), _headers_mtime()):
+    if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(src), _shared_mtime()):
         return obj
     cmd = [_nvcc(), *ARCH, *COMMON, "-c", src, "-o", obj]
     if src.endswith(".cpp"):
