@@ -125,7 +125,7 @@ typedef struct GbTuning {
     int32_t cmCtasPerSm, mqCtasPerSm, decCtasPerSm;
     int32_t t1Persistent;
     int32_t decHeavyPct;  /* Tier-1 decode: blocks whose codeword exceeds this % of the mean bytes per
-                             decoding warp run on SMs of their own, four per SM (0: none) */
+                             resident warp (24 an SM at most) run on SMs of their own, four per SM (0: none) */
     int32_t dwtTile1, dwtTileN;  /* encoder front-end tile at level 1 and at levels 2..: 0 = 64 x 64,
                                     1 = 128 x 64, 2 = 64 x 128 (same coefficients; read when an
                                     encoder or engine frame slot is made) */

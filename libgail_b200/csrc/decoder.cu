@@ -73,8 +73,8 @@ struct DecArgs {
     uint32_t W;
     uint32_t* perm;
     uint32_t* ctl;      // kCtlWords control words, zeroed before the launch
-    uint32_t slots;     // the decode launch's warps
-    uint32_t heavyPct;  // heavy: codeword bytes above heavyPct % of the mean per warp (0: none)
+    uint32_t slots;     // the decode launch's warps that are resident together
+    uint32_t heavyPct;  // heavy: codeword bytes above heavyPct % of the mean per such warp (0: none)
 };
 
 __device__ __forceinline__ uint32_t lenBucket(uint32_t len) {
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) orderScatterKernel(DecArgs a) {
             run += v[k];
         }
     }
-    // heavy blocks: above heavyPct % of the mean codeword bytes per decoding warp
+    // heavy blocks: above heavyPct % of the mean codeword bytes per resident warp
     const uint64_t limit = (uint64_t)a.ctl[4] * a.heavyPct / (100ull * max(a.slots, 1u));
     for (uint32_t first = blockIdx.x * 256u; first < a.n; first += gridDim.x * 256u) {
         const uint32_t i = first + tid;
@@ -918,7 +918,7 @@ void DecoderSlot::enqueue(const Layout& frame, const uint8_t* data, size_t size,
     const Tuning tu = tuningFor(L_.profile);
     const uint32_t grid = std::min<uint32_t>((uint32_t)n, (uint32_t)(sms * tu.decCtasPerSm));
     DecArgs da{dBytes_, size, dCodes_, dBlocks_, (uint32_t)n, dHalf_, (uint32_t*)dPlanes_, (uint32_t)L_.width, dPerm_, dCtl_,
-               grid, heavySms_ && alone ? (uint32_t)tu.decHeavyPct : 0u};
+               std::min(grid, (uint32_t)(sms * DEC_CTAS)), heavySms_ && alone ? (uint32_t)tu.decHeavyPct : 0u};
     const uint32_t og = std::max(1u, std::min(divUp((uint32_t)n, 256u), (uint32_t)sms * 2u));
     orderCountKernel<<<og, 256, 0, st>>>(da);
     orderScatterKernel<<<og, 256, 0, st>>>(da);
