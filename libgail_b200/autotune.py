@@ -16,6 +16,7 @@ from __future__ import annotations
 import argparse
 import ctypes as C
 import json
+import os
 import time
 
 import numpy as np
@@ -26,6 +27,7 @@ DEFAULTS = {"soloDecisions": 16384, "cmCtasPerSm": 16, "mqCtasPerSm": 16, "decCt
             "decHeavyPct": 150, "dwtTile1": 0, "dwtTileN": 0}
 POLICY_DEFAULT = {"maxBatch": 16, "minBatchPct": 25, "maxWaitMs": 2.0}
 PROFILES = {"2k": 0, "4k": 1}
+MARGIN = 0.04  # what a candidate has to gain: served rates of one configuration differ by 2-4 %
 
 
 class GbTuning(C.Structure):
@@ -60,12 +62,15 @@ def get_tuning(profile: int) -> dict:
     return {k: int(getattr(v, k)) for k in DEFAULTS}
 
 
-def coordinate_search(start: dict, space: dict, measure, rounds: int = 1, log=None):
+def coordinate_search(start: dict, space: dict, measure, rounds: int = 1, log=None, margin: float = 0.0):
     """Minimises measure(config) one knob at a time over its candidates (keeping the others),
-    `rounds` sweeps over the knobs. Returns (best config, its cost, every (config, cost))."""
+    `rounds` sweeps over the knobs; a candidate replaces the best so far only if it costs less by
+    more than `margin` of it. Returns (best config, its cost, every (config, cost))."""
     best = dict(start)
     best_cost = measure(best)
     seen = [(dict(best), best_cost)]
+    if log:
+        log(f"  as it is: {best_cost:.4f}")
     for _ in range(rounds):
         for knob, values in space.items():
             for v in values:
@@ -76,7 +81,7 @@ def coordinate_search(start: dict, space: dict, measure, rounds: int = 1, log=No
                 seen.append((dict(cand), cost))
                 if log:
                     log(f"  {knob}={v}: {cost:.4f}")
-                if cost < best_cost:
+                if cost < best_cost * (1.0 - margin):
                     best, best_cost = cand, cost
     return best, best_cost, seen
 
@@ -139,6 +144,17 @@ def _best_of(measure, runs: int):
     return lambda cfg: min(measure(cfg) for _ in range(runs))
 
 
+def _median_ms(burst, times: int = 15) -> float:
+    """The median wall time of a burst (how its frames fall into batches varies), after a first
+    one that warms up and makes what slots are missing."""
+    t = []
+    for _ in range(times + 1):
+        t0 = time.perf_counter()
+        burst()
+        t.append((time.perf_counter() - t0) * 1e3)
+    return float(np.median(t[1:]))
+
+
 def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
     import torch
 
@@ -152,6 +168,9 @@ def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
     dev = P.Plugin().device(0)
     out = {"device": torch.cuda.get_device_name(0), "sms": torch.cuda.get_device_properties(0).multi_processor_count,
            "profiles": {}, "policy": {}, "measured": {}}
+    policies = [dict(POLICY_DEFAULT, **p) for p in
+                ({}, {"maxBatch": 8}, {"maxBatch": 32}, {"minBatchPct": 10}, {"minBatchPct": 50})]
+    served = {name: [] for name in PROFILES}
     try:
         for name, prof in PROFILES.items():
             n = 4 if name == "4k" else 8
@@ -161,41 +180,35 @@ def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
             dframes = [torch.from_numpy(f.view(np.int16)).to("cuda:0") for f in frames]
             torch.cuda.synchronize()
             enc = dev.encoder(lay, fmt, col)
-            stage_ms = _stage_timer(L, enc, dframes, prof, n)  # plain one-frame launches
-
-            def tier1_ms(cfg):  # context modelling + MQ
-                return stage_ms(cfg, (1, 3))
+            stage_ms = _stage_timer(L, enc, dframes, prof, n)
 
             def front_ms(cfg):  # colour + wavelet + quantisation
                 return stage_ms(cfg, (0,))
 
             eng = Engine(0, 0, max_batch=POLICY_DEFAULT["maxBatch"])
             cid, _ = eng.add_encoder(lay, fmt, col)
-            eng.reserve(cid, len(dframes))  # a slot per frame of a burst before the first one
+            loads = dframes * 3  # several batches of the largest size
+            eng.reserve(cid, len(loads))  # a slot per frame of a burst before the first one
 
-            def served_ms(cfg):  # wall time per frame of a burst through the engine, Tier-1 only
+            def served_ms(cfg):  # wall time per frame of bursts through the engine, Tier-1 only
                 set_tuning(prof, cfg)
-                ids = [eng.submit(cid, f) for f in dframes[:n]]  # warm
-                for _ in ids:
-                    eng.release(eng.wait(120000, copy=False)[0])
-                t0 = time.perf_counter()
-                ids = [eng.submit(cid, f) for f in dframes]
-                for _ in ids:
-                    eng.release(eng.wait(120000, copy=False)[0])
-                return (time.perf_counter() - t0) * 1e3 / len(dframes)
+
+                def burst():
+                    ids = [eng.submit(cid, f) for f in loads]
+                    for _ in ids:
+                        eng.release(eng.wait(120000, copy=False)[0])
+                return _median_ms(burst) / len(loads)
 
             cfg = dict(DEFAULTS)
             log(f"[{name}] front-end tile shapes (front-end ms per frame)")
             tiles = {"dwtTile1": [1, 2], "dwtTileN": [1, 2]}
-            cfg, _, seen0 = coordinate_search(cfg, tiles, _best_of(front_ms, runs), log=log)
-            # one-frame launches use it in the persistent form only: their separate MQ launch
-            # has a rule of its own
-            log(f"[{name}] MQ solo threshold (Tier-1 ms per frame)")
-            solo = {"soloDecisions": [4096, 8192, 32768, 1 << 30]}
-            cfg, _, seen1 = coordinate_search(cfg, solo, _best_of(tier1_ms, runs), log=log)
-            log(f"[{name}] grid caps (served ms per frame)")
-            caps = {"cmCtasPerSm": [8, 12, 24], "mqCtasPerSm": [8, 12, 24], "t1Persistent": [1]}
-            cfg, _, seen2 = coordinate_search(cfg, caps, _best_of(served_ms, runs), log=log)
+            cfg, _, seen0 = coordinate_search(cfg, tiles, _best_of(front_ms, runs), log=log, margin=MARGIN)
+            # the solo threshold on batches, where it acts (a one-frame launch has a rule of its own),
+            # from the value the engine's batches take at least
+            log(f"[{name}] MQ solo threshold, grid caps (served ms per frame)")
+            caps = {"soloDecisions": [32768, 1 << 30], "cmCtasPerSm": [8, 12, 24], "mqCtasPerSm": [8, 12, 24],
+                    "t1Persistent": [1]}
+            cfg, _, seen2 = coordinate_search(cfg, caps, _best_of(served_ms, runs), log=log, margin=MARGIN)
             # the decoder's cap on this profile's own codestreams
             streams = []
             for f in frames[:2]:
@@ -204,18 +217,18 @@ def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
             # as decode requests to the engine, several in flight: the cap that serves most
             dcls, _ = eng.add_decoder(lay)
 
-            def decode_ms(c):  # wall time per decode of a burst through the engine
+            def decode_ms(c):  # wall time per decode of bursts through the engine
                 set_tuning(prof, c)
-                for rep in range(2):  # the first burst warms up (and makes the decoder slots)
-                    t0 = time.perf_counter()
+
+                def burst():
                     ids = [eng.submit_decode(dcls, s) for s in streams * 4]
                     for _ in ids:
                         eng.release(eng.wait(120000, copy=False)[0])
-                return (time.perf_counter() - t0) * 1e3 / len(ids)
+                return _median_ms(burst) / (4 * len(streams))
 
             log(f"[{name}] decoder grid cap (served decode ms per frame)")
             cfg, _, seen3 = coordinate_search(cfg, {"decCtasPerSm": [16, 24, 48, 64]}, _best_of(decode_ms, runs),
-                                             log=log)
+                                             log=log, margin=MARGIN)
             # the heavy-block threshold by one frame's Tier-1 decode on its own (the latency of
             # decoder_decode: the longest codewords' serial chains set it)
             blocks = [CS.parse(s)[1].view(P.CBLK_CODE_DTYPE) for s in streams]
@@ -224,34 +237,30 @@ def tune(quick: bool = False, log=print, runs: int = 2) -> dict:
 
             def decode_t1_ms(c):
                 set_tuning(prof, c)
-                t = []
-                for s, b in zip(streams, blocks):
-                    dec.decode(s, b, out=pic)
-                    t.append(dec.decode(s, b, out=pic)[1].t1)
-                return float(np.mean(t))
+                t = [[dec.decode(s, b, out=pic)[1].t1 for _ in range(12)] for s, b in zip(streams, blocks)]
+                return float(np.mean(np.median(np.array(t)[:, 2:], axis=1)))
 
             log(f"[{name}] decoder heavy-block threshold (Tier-1 decode ms of one frame)")
-            cfg, _, seen5 = coordinate_search(cfg, {"decHeavyPct": [0, 150, 400, 800]}, _best_of(decode_t1_ms, runs),
-                                             log=log)
+            cfg, _, seen5 = coordinate_search(cfg, {"decHeavyPct": [0, 100, 200, 400, 800]},
+                                             _best_of(decode_t1_ms, runs), log=log, margin=MARGIN)
             seen3 = seen3 + seen5
             dec.close()
-            if name == "4k":
-                log("[4k] engine batch policy (served ms per frame)")
-                pol = dict(POLICY_DEFAULT)
-
-                def policy_ms(p):
-                    eng.set_policy(p["maxBatch"], p["minBatchPct"], p["maxWaitMs"])
-                    return served_ms(cfg)
-
-                space = {"maxBatch": [8, 32], "minBatchPct": [10, 50]}
-                pol, _, seen4 = coordinate_search(pol, space, _best_of(policy_ms, runs), log=log)
-                out["policy"] = pol
-                out["measured"]["policy"] = [[c, round(v, 4)] for c, v in seen4]
+            # the batch policy with codestreams, as it is served, on both profiles' frames
+            log(f"[{name}] engine batch policy (served codestreams, ms per frame)")
+            eng.set_codestream(fps=24.0, tag="tune", threads=max(2, min(12, (os.cpu_count() or 4) - 2)))
+            for p in policies:
+                eng.set_policy(p["maxBatch"], p["minBatchPct"], p["maxWaitMs"])
+                served[name].append(min(served_ms(cfg) for _ in range(runs)))
+                log(f"  {p['maxBatch']}, {p['minBatchPct']} %: {served[name][-1]:.4f}")
             eng.close()
             enc.close()
             out["profiles"][name] = cfg
-            out["measured"][name] = [[c, round(v, 4)] for c, v in seen0 + seen1 + seen2 + seen3]
+            out["measured"][name] = [[c, round(v, 4)] for c, v in seen0 + seen2 + seen3]
             set_tuning(prof, None)
+        # against the default's time on the same frames, both profiles alike
+        cost = [float(np.mean([served[n][i] / served[n][0] for n in served])) for i in range(len(policies))]
+        out["policy"] = policies[int(np.argmin(cost))]
+        out["measured"]["policy"] = [[p, {n: round(served[n][i], 4) for n in served}] for i, p in enumerate(policies)]
     finally:
         dev.close()
     return out

@@ -42,6 +42,12 @@ def test_coordinate_search_finds_the_minimum():
     assert len(seen) == 1 + 4 + 3
 
 
+def test_a_candidate_has_to_gain_more_than_the_margin():
+    noise = iter([1.0, 0.995, 0.99, 0.985, 1.01, 0.97])
+    best, c, _ = AT.coordinate_search({"a": 0}, {"a": [1, 2, 3, 4, 5]}, lambda cfg: next(noise), margin=0.02)
+    assert best == {"a": 5} and c == 0.97  # those within the noise do not replace the default
+
+
 def test_apply_only_on_the_same_gpu(tmp_path):
     f = tmp_path / "t.json"
     f.write_text(json.dumps({"device": "NVIDIA B200", "profiles": {"4k": dict(AT.DEFAULTS, mqCtasPerSm=12)},
