@@ -1,5 +1,6 @@
 """MQ coding against the C oracle at the sizes where its launch changes (every block alone in a
-warp, some alone, more blocks than a warp per scheduler takes, a batched launch's kernel), with
+warp, some alone, more blocks than a warp per scheduler takes, the last with one warp per scheduler
+and the first with two (148 SMs), a batched launch's kernel), with
 blocks of a few decisions to thousands and enough bytes that carries meet 0xFF bytes. Bytes and
 whole numbers, so everything is compared exactly."""
 import numpy as np
@@ -10,7 +11,8 @@ from oracle.oracle import Oracle
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,size,planes", [(1, 32, 12), (33, 32, 14), (700, 32, 9), (18900, 8, 12), (19000, 8, 12), (76000, 8, 9)])
+@pytest.mark.parametrize("n,size,planes", [(1, 32, 12), (33, 32, 14), (700, 32, 9), (18900, 8, 12), (19000, 8, 12), (28416, 4, 9),
+                                           (28417, 8, 9), (52000, 4, 9), (76000, 8, 9)])
 def test_mq_matches_oracle(n, size, planes):
     rng = np.random.default_rng(n)
     top = 1 << (planes + 6)
