@@ -114,7 +114,8 @@ GB_API int gb_color_route(const GailCudaColor* color, float* params48, int32_t* 
  *   soloDecisions  MQ coding in launches of more than 128 blocks per scheduler (75,776 on
  *                  148 SMs): blocks with at least this many decisions are coded alone in a
  *                  warp first (rounded down to a power of two; default 16384). Smaller
- *                  launches run a warp per scheduler and code their longest blocks alone.
+ *                  launches run one warp per scheduler, two above 48 blocks per scheduler
+ *                  (28,416), and code their longest blocks alone.
  *   cmCtasPerSm, mqCtasPerSm, decCtasPerSm  grid caps in CTAs per SM of context modelling,
  *                  MQ coding (such launches) and Tier-1 decoding (defaults 16, 16, 32; 1..64)
  *   t1Persistent   1: Tier-1 encoding as one persistent launch whose warps take context

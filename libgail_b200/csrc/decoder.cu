@@ -49,7 +49,7 @@ __constant__ uint8_t c_sc[9];
 __constant__ uint32_t c_mq[47];
 
 // Heavy blocks: the longest codewords, decoded on SMs of their own (at most four per SM, one
-// per scheduler) instead of beside 31 other decoding warps, where a block of a thousand
+// per scheduler) instead of beside 23 other decoding warps, where a block of a thousand
 // bytes or more takes the whole launch's time.
 constexpr uint32_t kMaxReserveSms = 32;
 constexpr uint32_t kMaxHeavy = 4 * kMaxReserveSms;
@@ -729,9 +729,10 @@ constexpr size_t kInvSmem = (size_t)TW * TP * 4;
 }  // namespace
 
 void decoderInit() {
-    uint8_t zc[4 * 45], sc[9];
+    uint8_t sc[9];
     uint32_t mq[47];
-    t1BuildTables(zc, sc, mq);
+    signTable(sc);
+    mqTable(mq);
     GB_CHECK(cudaMemcpyToSymbol(c_sc, sc, sizeof sc));
     GB_CHECK(cudaMemcpyToSymbol(c_mq, mq, sizeof mq));
     GB_CHECK(cudaFuncSetAttribute(invLevelKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmemLast));

@@ -377,10 +377,12 @@ __device__ __forceinline__ uint32_t orderBucket(uint32_t s) {
     return ORDER_BUCKETS - 1 - cls;
 }
 
-// Blocks with at least P.soloDecisions decisions are MQ-coded alone in a warp (its lane 0),
-// at most one per warp for half the launch's warps: the longest serial chains, which would
-// otherwise run beside 31 divergent neighbours. A power of two, so that they are exactly
-// the first blocks of the order.
+// The first blocks of the order are MQ-coded alone in a warp (its lane 0), one per warp at most: the
+// longest serial chains, which would otherwise run beside 31 neighbours. As many as have
+// P.soloDecisions decisions or more, up to maxSolo: half the warps of a batched launch, whose
+// soloDecisions is a power of two and so the limit of a class; up to every warp of a smaller one,
+// whose soloDecisions is 1 (the last class holds blocks without a decision too: a warp that gets
+// one goes on at once).
 __global__ void __launch_bounds__(1024) t1OrderKernel(T1Launch P, uint32_t maxSolo) {
     __shared__ uint32_t hist[ORDER_BUCKETS];
     __shared__ uint32_t solo;
@@ -624,9 +626,9 @@ __device__ __forceinline__ void mqTables(uint2* s_next, uint32_t* s_init) {
 // null context, so every lane of the warp takes the same 16 steps. The bytes are taken out
 // after them, where a byte completed in the middle of a decision made nearly every decision
 // of a warp take the byte's branch as well. A round sets up 32 decisions (16 at a time: 3-5 %
-// slower). On a B200, per 4K frame (154 M decisions): 1.11 ms alone where the coder with the
-// branch took 2.21, 0.50 ms of a batch of eight; the 48 blocks of a 64 x 64 frame 0.48 ms,
-// where they took 1.35. CHAIN: the form with the shorter chain and a few more instructions,
+// slower). On a B200, per 4K frame (154 M decisions): 0.95 ms alone (1.11 with a lane for every
+// block) where the coder with the branch took 2.21, 0.50 ms of a batch of eight; the 48 blocks of a
+// 64 x 64 frame 0.48 ms, where they took 1.35. CHAIN: the form with the shorter chain and a few more instructions,
 // for one-frame launches (1.15 against 1.18 ms).
 template <int CS, bool PERS, bool CHAIN>
 __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* s_mq, uint32_t lane0, const uint2* s_next,
@@ -856,7 +858,7 @@ __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* s_mq, uint32_
 
 // MINB: CTAs per SM the registers must allow. A launch of a frame or two has fewer lanes
 // than the GPU holds and runs uncapped; wide batched launches run at 6 CTAs per SM (24 frames
-// of 4K served on a B200: 33.6 ms, 34.3 at 8 CTAs; 10 would spill).
+// of 4K served on a B200: 30.5 ms, 2 % more at 8 CTAs; 10 would spill).
 template <int MINB>
 __global__ void __launch_bounds__(MQ_THREADS, MINB) t1MqKernel(T1Launch P) {
     __shared__ uint2 s_next[128];
@@ -1094,9 +1096,8 @@ cudaError_t kernelsLoadable() {
 }
 
 void t1Init() {
-    uint8_t zc[4 * 45], sc[9];
     uint32_t mq[47];
-    t1BuildTables(zc, sc, mq);
+    mqTable(mq);
     GB_CHECK(cudaMemcpyToSymbol(c_mq, mq, sizeof mq));
 }
 

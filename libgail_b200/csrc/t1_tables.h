@@ -1,31 +1,10 @@
-// Context and probability tables of EBCOT Tier-1 (ISO/IEC 15444-1 Tables C.2, D.1 and
-// D.3), built on the host in the packed forms the kernels index.
+// Sign-coding and probability tables of EBCOT Tier-1 (ISO/IEC 15444-1 Tables D.3 and C.2), built on
+// the host in the packed forms the kernels index (zero-coding contexts, Table D.1, are boolean
+// forms in t1_masks.cuh).
 #pragma once
 #include <cstdint>
 
 namespace gb {
-
-// Zero-coding context from the counts of significant horizontal (h, 0..2), vertical
-// (v, 0..2) and diagonal (d, 0..4) neighbours; orient 0 LL, 1 HL, 2 LH, 3 HH (Table D.1).
-inline int zcContext(int h, int v, int d, int orient) {
-    if (orient == 3) {
-        const int hv = h + v;
-        if (d >= 3) return 8;
-        if (d == 2) return hv >= 1 ? 7 : 6;
-        if (d == 1) return hv >= 2 ? 5 : (hv == 1 ? 4 : 3);
-        return hv >= 2 ? 2 : hv;
-    }
-    if (orient == 1) {  // the horizontally high-pass band swaps the roles of h and v
-        const int t = h;
-        h = v;
-        v = t;
-    }
-    if (h == 2) return 8;
-    if (h == 1) return v >= 1 ? 7 : (d >= 1 ? 6 : 5);
-    if (v == 2) return 4;
-    if (v == 1) return 3;
-    return d >= 2 ? 2 : d;
-}
 
 // Sign-coding context and XOR bit from the clamped horizontal and vertical sign
 // contributions hc, vc in -1..1 (Table D.3).
@@ -61,20 +40,18 @@ inline const MqState* mqStates() {
     return t;
 }
 
-// zc: 4 x 45 bytes indexed by orient * 45 + h + 3 v + 9 d; sc: 9 bytes indexed by
-// (hc + 1) * 3 + (vc + 1), context | xor << 5; mq: 47 words Qe | switch << 17 |
-// NMPS << 18 | NLPS << 24 (bit 16 is left for the context's MPS).
-inline void t1BuildTables(uint8_t* zc, uint8_t* sc, uint32_t* mq) {
-    for (int o = 0; o < 4; ++o)
-        for (int d = 0; d <= 4; ++d)
-            for (int v = 0; v <= 2; ++v)
-                for (int h = 0; h <= 2; ++h) zc[o * 45 + h + 3 * v + 9 * d] = (uint8_t)zcContext(h, v, d, o);
+// 9 bytes indexed by (hc + 1) * 3 + (vc + 1): context | xor << 5.
+inline void signTable(uint8_t* sc) {
     for (int hc = -1; hc <= 1; ++hc)
         for (int vc = -1; vc <= 1; ++vc) {
             int cx, x;
             scContext(hc, vc, cx, x);
             sc[(hc + 1) * 3 + (vc + 1)] = (uint8_t)(cx | (x << 5));
         }
+}
+
+// 47 words Qe | switch << 17 | NMPS << 18 | NLPS << 24.
+inline void mqTable(uint32_t* mq) {
     const MqState* s = mqStates();
     for (int i = 0; i < 47; ++i)
         mq[i] = (uint32_t)s[i].qe | ((uint32_t)s[i].sw << 17) | ((uint32_t)s[i].nmps << 18) | ((uint32_t)s[i].nlps << 24);
