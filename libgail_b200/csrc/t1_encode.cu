@@ -764,8 +764,8 @@ __device__ __forceinline__ void mqRun(const T1Launch& P, uint32_t* s_mq, uint32_
         // one (it and the three bits below read 0 after a carry), and a round of more shifts
         // than the register holds, are done over from the steps, byte by byte.
         const Coder before = e;
-        int left = (int)shift;
         bool redo = shift > 32u;
+        int left = redo ? 0 : (int)shift;
         uint32_t keep = 0xFFFFFFFFu;
         while (left >= e.CT) {
             left -= e.CT;
