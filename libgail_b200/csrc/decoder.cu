@@ -362,21 +362,13 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decodeKernel(DecArgs a)
                                           (d.right << 1) | (d.right >> 1);
                     uint32_t m[8] = {nAny & ~d.refined, d.refined, 0u, 0u, 0u, 0u, 0u, 0u};
                     rowBytes(m);
-                    const uint32_t c = nibbleCounts(E);
-                    const uint32_t w0 = (c & 0xFu) | (((c >> 4) & 0xFu) << 10) | (((c >> 8) & 0xFu) << 20);
-                    const uint32_t w1 = ((c >> 12) & 0xFu) | (((c >> 16) & 0xFu) << 10) | (((c >> 20) & 0xFu) << 20);
-                    const uint32_t w2 = ((c >> 24) & 0xFu) | ((c >> 28) << 10);
-                    const uint32_t i0 = warpScan(w0, lane), i1 = warpScan(w1, lane), i2 = warpScan(w2, lane);
-                    const uint32_t x0 = i0 - w0, x1 = i1 - w1, x2 = i2 - w2;
-                    const uint32_t t0 = __shfl_sync(kFull, i0, 31), t1 = __shfl_sync(kFull, i1, 31),
-                                   t2 = __shfl_sync(kFull, i2, 31);
+                    const StripePlaces places(nibbleCounts(E), lane);
                     uint32_t total = 0;
                     uint8_t* list = reinterpret_cast<uint8_t*>(s_list);
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
-                        const int sh = 10 * (s % 3);
-                        uint8_t* o = list + total + (((s < 3 ? x0 : (s < 6 ? x1 : x2)) >> sh) & 1023u);
-                        total += ((s < 3 ? t0 : (s < 6 ? t1 : t2)) >> sh) & 1023u;
+                        uint8_t* o = list + total + places.before(s);
+                        total += places.all(s);
                         uint32_t z = m[s];
 #pragma unroll
                         for (int i = 0; i < 4; ++i, z >>= 8)
@@ -420,9 +412,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_CTAS) decodeKernel(DecArgs a)
                     total = 0;
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
-                        const int sh = 10 * (s % 3);
-                        const uint32_t at = total + (((s < 3 ? x0 : (s < 6 ? x1 : x2)) >> sh) & 1023u);
-                        total += ((s < 3 ? t0 : (s < 6 ? t1 : t2)) >> sh) & 1023u;
+                        const uint32_t at = total + places.before(s);
+                        total += places.all(s);
                         uint32_t bits = __funnelshift_r(s_bits[at >> 5], s_bits[(at >> 5) + 1], at & 31u);
 #pragma unroll
                         for (int i = 0; i < 4; ++i)

@@ -278,22 +278,16 @@ __device__ __forceinline__ uint32_t cmJob(const T1Launch& P, uint32_t job, uint3
                     for (int k = 0; k < kFracBits; ++k) dist += (192 << k) * __popc(NEW & planes[p + k][lane]);
                 }
                 total = __reduce_add_sync(kFull, dist);
-                // (3) decisions per stripe, 10-bit fields, three stripes per word, and each
-                //     lane's place among them
+                // (3) decisions per stripe, and each lane's place among them
                 const uint32_t c = nibbleCounts(EZ) + nibbleCounts(NEW) + runs + 2u * newRun;
-                const uint32_t w0 = (c & 0xFu) | (((c >> 4) & 0xFu) << 10) | (((c >> 8) & 0xFu) << 20);
-                const uint32_t w1 = ((c >> 12) & 0xFu) | (((c >> 16) & 0xFu) << 10) | (((c >> 20) & 0xFu) << 20);
-                const uint32_t w2 = ((c >> 24) & 0xFu) | ((c >> 28) << 10);
-                const uint32_t i0 = warpScan(w0, lane), i1 = warpScan(w1, lane), i2 = warpScan(w2, lane);
-                uint32_t x0 = i0 - w0, x1 = i1 - w1, x2 = i2 - w2;
-                uint32_t t0 = __shfl_sync(kFull, i0, 31), t1 = __shfl_sync(kFull, i1, 31), t2 = __shfl_sync(kFull, i2, 31);
+                const StripePlaces places(c, lane);
                 // (4) every lane writes its decisions, stripe after stripe
                 uint32_t before = count;  // decisions of the pass's stripes so far
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
-                    const int r0 = 4 * s, sh = 10 * (s % 3);
-                    uint8_t* o = pb + before + (((s < 3 ? x0 : (s < 6 ? x1 : x2)) >> sh) & 1023u);
-                    before += ((s < 3 ? t0 : (s < 6 ? t1 : t2)) >> sh) & 1023u;
+                    const int r0 = 4 * s;
+                    uint8_t* o = pb + before + places.before(s);
+                    before += places.all(s);
                     if (type == 1) {
                         uint32_t z = m[s];
 #pragma unroll

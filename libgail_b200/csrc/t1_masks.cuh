@@ -99,6 +99,25 @@ __device__ __forceinline__ void rowBytes(uint32_t m[8]) {
     for (int k = 0; k < 8; ++k) m[k] = t[k];
 }
 
+// The places of a pass's decisions, stripe by stripe and column by column: from c, a lane's decisions
+// per stripe as 4-bit groups (15 at most), the decisions before the lane's in its stripe and the
+// stripe's in all columns. Counts are 10-bit fields, three stripes a word.
+struct StripePlaces {
+    uint32_t x[3], t[3];
+    __device__ __forceinline__ StripePlaces(uint32_t c, int lane) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t w = ((c >> (12 * k)) & 0xFu) | (((c >> (12 * k + 4)) & 0xFu) << 10) |
+                               (k < 2 ? ((c >> (12 * k + 8)) & 0xFu) << 20 : 0u);
+            const uint32_t incl = warpScan(w, lane);
+            x[k] = incl - w;
+            t[k] = __shfl_sync(kFull, incl, 31);
+        }
+    }
+    __device__ __forceinline__ uint32_t before(int s) const { return (x[s / 3] >> (10 * (s % 3))) & 1023u; }
+    __device__ __forceinline__ uint32_t all(int s) const { return (t[s / 3] >> (10 * (s % 3))) & 1023u; }
+};
+
 // Bit i of x (x < 16) to bit 0 of byte i, by one multiply: the four shifted copies of x land in
 // disjoint bit ranges.
 __device__ __forceinline__ uint32_t spread1(uint32_t x) { return (x * 0x00204081u) & 0x01010101u; }
