@@ -154,8 +154,8 @@ GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uin
         DeviceParts d;
         const size_t tables = (size_t)n * kMaxPasses * 4;
         const size_t oCoeffs = d.add((size_t)n * kCblkArea * 4), oJobs = d.add(n * sizeof(T1Job)), oInfo = d.add(16 * (size_t)n),
-                     oEnd = d.add(tables), oLen = d.add(tables), oDist = d.add(tables), oSnaps = d.add(4 * tables),
-                     oPerm = d.add(4 * (size_t)n), oCtl = d.add(64), oSlope = d.add(4), oOutInfo = d.add(20 * (size_t)n),
+                     oEnd = d.add(tables), oLen = d.add(tables), oDist = d.add(tables), oCtl = d.add(64),
+                     oSnaps = d.add(4 * tables), oPerm = d.add(4 * (size_t)n), oSlope = d.add(4), oOutInfo = d.add(20 * (size_t)n),
                      oOffsets = d.add(8 * (size_t)n), oSym = d.add(region), oCw = d.add(region);
         d.make();
         for (uint32_t i = 0; i < n; ++i) {
@@ -167,10 +167,9 @@ GB_API int gb_t1_encode_blocks(const uint32_t* coeffs, const int32_t* geom4, uin
         GB_CHECK(cudaMemcpy(d.at<void>(oCoeffs), coeffs, (size_t)n * kCblkArea * 4, cudaMemcpyHostToDevice));
         GB_CHECK(cudaMemcpy(d.at<void>(oJobs), jobs.data(), n * sizeof(T1Job), cudaMemcpyHostToDevice));
         GB_CHECK(cudaMemcpy(d.at<void>(oSlope), &slope, 4, cudaMemcpyHostToDevice));
-        GB_CHECK(cudaMemset(d.at<void>(oCtl), 0, 64));
-        // the kernels write a block's passes alone; the rest of its rows is 0, not what a call before left
-        GB_CHECK(cudaMemset(d.at<void>(oLen), 0, tables));
-        GB_CHECK(cudaMemset(d.at<void>(oDist), 0, tables));
+        // the control words, and before them the pass tables: the kernels write a block's passes alone,
+        // and the rest of its rows is 0, not what a call before left
+        GB_CHECK(cudaMemset(d.at<void>(oLen), 0, oCtl + 64 - oLen));
         uint32_t* const ctl = d.at<uint32_t>(oCtl);
         T1Launch L{d.at<T1Job>(oJobs), n, d.at<uint32_t>(oInfo), d.at<uint32_t>(oEnd), d.at<uint32_t>(oLen),
                    d.at<int32_t>(oDist), d.at<uint4>(oSnaps), d.at<uint32_t>(oPerm), ctl, d.at<float>(oSlope)};
